@@ -589,6 +589,7 @@ int fft3d_batch_step(fft3d_batch* b, int count, fft3d_plane* const* planes, cons
       run.r.a = d.inv[i].a;
       for (auto& p : run.r.a.in) p = nullptr;
       run.r.ts.count = (int)(e - i);
+      run.r.ts.nb = 1;
       for (size_t k = i; k < e; k++) {
         for (int w = 0; w < 5; w++)
           if (d.inv[k].a.in[w]) run.r.ts.spec[(k - i) + w] = d.inv[k].a.in[w];

@@ -156,6 +156,7 @@ struct TemporalSet {
   const float2* spec[kGroupTile + 4];
   float* tdom[kGroupTile];
   int count;
+  int nb;  // consecutive blocks per CTA (set by the launcher; 1 in batched runs)
 };
 
 // One run of a batched step's frame groups (work items: its plane's blocks).

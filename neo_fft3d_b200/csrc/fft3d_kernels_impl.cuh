@@ -26,6 +26,9 @@ constexpr int kWarps = 4;       // warps per CTA in k_forward / k_filter_inverse
 #ifndef FFT3D_GROUP_CTAS
 #define FFT3D_GROUP_CTAS 6
 #endif
+// ... and for short Wiener 3D runs, whose threads hold two windows (the one
+// they filter and the next one's loads in flight)
+constexpr int kShortCtas = 5;
 // forward rows of a lane walked by a loop (one copy of the row code) instead
 // of unrolled: fewer instruction-cache misses, the forward's largest stall
 // (measured at 1080p bw=32: 22.0 vs 23.5 us per frame over all planes)
@@ -344,7 +347,7 @@ __device__ __forceinline__ void store_tdom(const float2* Sb, float* out, int lan
 template <int BW, int BH, typename T, bool PREFETCH, class Win>
 __device__ __forceinline__ void forward_cta_w(const ForwardArgs& a, int cta, const Win& win) {
   constexpr int NH = BW / 2 + 1, HC = BW / 2, NBW = blocks_per_warp<BW>(), BINS = BH * NH;
-  extern __shared__ float2 smem2[];
+  extern __shared__ __align__(16) float2 smem2[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* S = smem2 + warp * NBW * BINS;
   const Geom& g = a.g;
@@ -692,6 +695,219 @@ __device__ __forceinline__ float2 sharpen_bin(const InverseArgs& a, float2 v, co
   return __ffma2_rn(c, make_float2(f, f), gc);
 }
 
+// ---------------------------------------------------------------- filters, two bins at a time
+
+// Two floats in one 64-bit register pair, for the packed f32x2 instructions
+// (each lane rounds like the scalar operation). Held as one 64-bit value and
+// worked on with PTX: the same arithmetic on float2 and its intrinsics cost 50
+// register moves per bin pair and frame at bt = 5 (188 instructions instead of
+// 128), because the halves are then allocated one by one.
+using f2x = unsigned long long;
+__device__ __forceinline__ f2x pk2(float lo, float hi) {
+  f2x r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f2x dup2(float v) { return pk2(v, v); }
+__device__ __forceinline__ float2 up2(f2x v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2x add2(f2x a, f2x b) {
+  f2x r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2x sub2(f2x a, f2x b) {
+  f2x r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2x mul2(f2x a, f2x b) {
+  f2x r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2x fma2(f2x a, f2x b, f2x c) {
+  f2x r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2x rcp2(f2x v) {
+  const float2 u = up2(v);
+  return pk2(rcp_nrm(u.x), rcp_nrm(u.y));
+}
+__device__ __forceinline__ f2x max2(f2x v, float w) {
+  const float2 u = up2(v);
+  return pk2(fmaxf(u.x, w), fmaxf(u.y, w));
+}
+
+// Two neighbouring bins: their real parts and their imaginary parts, packed.
+// The filter's arithmetic is the same for both bins, so every sum, product
+// and fused multiply-add of the pair is one instruction, the turns by -i cost
+// nothing (re and im change places), and the pair's Wiener factors come as a
+// packed value that scales both parts. A pair gives what filter_vals and
+// sharpen_bin give for its two bins, bit for bit.
+struct Pair {
+  f2x re, im;
+};
+// The filter's constants as pairs, read from the constant bank by the packed
+// instructions.
+__constant__ float2 c_pair[] = {
+    {0.30901699437494742410229341718282f, 0.30901699437494742410229341718282f},    // kCos72
+    {-0.80901699437494742410229341718282f, -0.80901699437494742410229341718282f},  // kCos144
+    {0.95105651629515357211643933337938f, 0.95105651629515357211643933337938f},    // kSin72
+    {0.58778525229247312916870595463907f, 0.58778525229247312916870595463907f},    // kSin144
+    {-0.58778525229247312916870595463907f, -0.58778525229247312916870595463907f},  // kMinusSin144
+    {0.86602540378443864676372317075294f, 0.86602540378443864676372317075294f},    // kSin120
+    {-0.5f, -0.5f},                                                                // kMinusHalf
+    {1.0e-15f, 1.0e-15f},                                                          // kPsdFloor
+    {1.f, 1.f},                                                                    // kOne
+    {0.5f, 0.5f},                                                                  // kHalf
+    {1.0f / 3.0f, 1.0f / 3.0f},                                                    // kThird
+    {0.25f, 0.25f},                                                                // kQuarter
+    {0.2f, 0.2f},                                                                  // kFifth
+};
+enum PairConst { kCos72, kCos144, kSin72, kSin144, kMinusSin144, kSin120, kMinusHalf, kPsdFloor, kOne, kHalf, kThird, kQuarter, kFifth };
+__device__ __forceinline__ f2x kc(PairConst k) { return reinterpret_cast<const f2x*>(c_pair)[k]; }
+
+__device__ __forceinline__ Pair pair_of(const float4& v) { return Pair{pk2(v.x, v.z), pk2(v.y, v.w)}; }
+__device__ __forceinline__ float4 bins_of(const Pair& p) {
+  const float2 re = up2(p.re), im = up2(p.im);
+  return make_float4(re.x, im.x, re.y, im.y);
+}
+__device__ __forceinline__ Pair padd(const Pair& x, const Pair& y) { return Pair{add2(x.re, y.re), add2(x.im, y.im)}; }
+// x * s with products that stay products: ptxas contracts a packed multiply
+// into a packed add that follows (explicit rounding or not), which would round
+// once where filter_vals and sharpen_bin round twice; two scalar multiplies
+// are left alone, at the same cost on the FMA pipe.
+__device__ __forceinline__ f2x mul2_kept(f2x v, f2x s) {
+  const float2 a = up2(v), b = up2(s);
+  return pk2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+}
+__device__ __forceinline__ Pair pscale_kept(const Pair& x, f2x s) { return Pair{mul2_kept(x.re, s), mul2_kept(x.im, s)}; }
+__device__ __forceinline__ Pair psub(const Pair& x, const Pair& y) { return Pair{sub2(x.re, y.re), sub2(x.im, y.im)}; }
+__device__ __forceinline__ Pair pscale(const Pair& x, f2x s) { return Pair{mul2(x.re, s), mul2(x.im, s)}; }
+__device__ __forceinline__ Pair pfma(const Pair& x, f2x s, const Pair& y) { return Pair{fma2(x.re, s, y.re), fma2(x.im, s, y.im)}; }
+// x - i v and x + i v
+__device__ __forceinline__ Pair psub_i(const Pair& x, const Pair& v) { return Pair{add2(x.re, v.im), sub2(x.im, v.re)}; }
+__device__ __forceinline__ Pair padd_i(const Pair& x, const Pair& v) { return Pair{sub2(x.re, v.im), add2(x.im, v.re)}; }
+__device__ __forceinline__ f2x ppsd(const Pair& v) { return fma2(v.re, v.re, fma2(v.im, v.im, kc(kPsdFloor))); }
+// The factors of wiener() for both bins; nn: minus their noise powers. The
+// parts scaled by them are summed with fused multiply-adds, as the compiler
+// contracts filter_vals' sums: fma(x, fx, y fy) for x fx + y fy.
+__device__ __forceinline__ f2x pfactor(const Pair& v, f2x nn, float lowlimit) {
+  return max2(fma2(nn, rcp2(ppsd(v)), kc(kOne)), lowlimit);
+}
+__device__ __forceinline__ Pair psum2(const Pair& x, f2x fx, const Pair& y, f2x fy) { return pfma(x, fx, pscale(y, fy)); }
+
+// filter_vals of a Wiener 3D mode for a pair; w: the pair in the window's
+// frames, grid: the pair's gridsample (zeros without degrid), gf: the block's
+// grid fraction, nn: minus the pair's noise powers.
+template <int MODE>
+__device__ __forceinline__ Pair filter_pair(const Pair (&w)[5], const Pair& grid, float gf, f2x nn, float ll) {
+  static_assert(MODE >= 2 && MODE <= 5, "Wiener 3D");
+  const Pair cur = w[2], g = pscale_kept(grid, dup2(gf * (float)MODE));
+  auto factor = [&](const Pair& v) { return pfactor(v, nn, ll); };
+  if constexpr (MODE == 2) {
+    const Pair f0 = psub(padd(cur, w[1]), g), f1 = psub(cur, w[1]);
+    return pscale(padd(psum2(f0, factor(f0), f1, factor(f1)), g), kc(kHalf));
+  } else if constexpr (MODE == 3) {
+    const Pair pn = padd(w[1], w[3]);
+    const Pair fc = psub(padd(cur, pn), g);
+    const Pair h = pfma(pn, kc(kMinusHalf), cur), d = pscale_kept(psub(w[1], w[3]), kc(kSin120));
+    const Pair fp = psub_i(h, d), fn = padd_i(h, d);
+    return pscale(padd(pfma(fn, factor(fn), psum2(fc, factor(fc), fp, factor(fp))), g), kc(kThird));
+  } else if constexpr (MODE == 4) {
+    const Pair cp = padd(cur, w[0]), cm = psub(cur, w[0]), pn = padd(w[1], w[3]), d = psub(w[1], w[3]);
+    const Pair fp2 = psub(cp, pn), fc = psub(padd(cp, pn), g);
+    const Pair fp = psub_i(cm, d), fn = padd_i(cm, d);
+    return pscale(padd(padd(psum2(fp2, factor(fp2), fp, factor(fp)), psum2(fc, factor(fc), fn, factor(fn))), g),
+                  kc(kQuarter));
+  } else {
+    const Pair a2 = padd(w[0], w[4]), a1 = padd(w[1], w[3]);
+    const Pair e2 = psub(w[4], w[0]), e1 = psub(w[1], w[3]);
+    const Pair s1 = padd(pfma(a2, kc(kCos72), pscale(a1, kc(kCos144))), cur);
+    const Pair s2 = padd(pfma(a2, kc(kCos144), pscale(a1, kc(kCos72))), cur);
+    const Pair t1 = pfma(e2, kc(kSin72), pscale(e1, kc(kSin144)));
+    const Pair t2 = pfma(e2, kc(kMinusSin144), pscale(e1, kc(kSin72)));
+    const Pair fp2 = psub_i(s1, t1), fn2 = padd_i(s1, t1);
+    const Pair fp = psub_i(s2, t2), fn = padd_i(s2, t2);
+    const Pair fc = psub(padd(padd(a2, a1), cur), g);
+    const Pair sum = padd(psum2(fp2, factor(fp2), fp, factor(fp)), psum2(fc, factor(fc), fn, factor(fn)));
+    return pscale(padd(pfma(fn2, factor(fn2), sum), g), kc(kFifth));
+  }
+}
+
+// sharpen_bin of a pair; wsh, wdh: the pair's weights.
+__device__ __forceinline__ Pair sharpen_pair(const InverseArgs& a, const Pair& v, const Pair& grid, f2x wsh, f2x wdh,
+                                             float gf) {
+  const Pair gc = pscale_kept(grid, dup2(gf)), c = psub(v, gc);
+  const f2x psd = ppsd(c);
+  f2x f = kc(kOne);
+  if (a.c.use_sharpen) {
+    const f2x smax = dup2(a.c.smax2n);
+    const f2x r = mul2(mul2(psd, smax), rcp2(mul2(add2(psd, dup2(a.c.smin2n)), add2(psd, smax))));
+    const float2 m = up2(max2(r, 1e-30f));
+    f = fma2(mul2(dup2(a.c.sharpen), wsh), mul2(r, pk2(rsqrt_nrm(m.x), rsqrt_nrm(m.y))), kc(kOne));
+  }
+  if (a.c.use_dehalo || !a.c.use_sharpen) {
+    const f2x top = add2(psd, dup2(a.c.ht2n));
+    const f2x d = mul2(top, rcp2(fma2(mul2(dup2(a.c.dehalo), wdh), psd, top)));
+    f = a.c.use_sharpen ? mul2(f, d) : d;
+  }
+  return Pair{fma2(c.re, f, gc.re), fma2(c.im, f, gc.im)};
+}
+
+// The gridsample of bins bin, bin + 1, or zeros without degrid.
+__device__ __forceinline__ Pair pair_grid(const InverseArgs& a, int bin) {
+  if (a.c.degrid == 0.f) return Pair{0, 0};
+  return pair_of(__ldg(reinterpret_cast<const float4*>(a.t.grid + bin)));
+}
+// Minus the noise powers of bins bin, bin + 1 of the block at `off`.
+template <int MODE>
+__device__ __forceinline__ f2x pair_noise(const InverseArgs& a, size_t off, int bin) {
+  if (a.psd) return pk2(-learned_noise(a, off, bin), -learned_noise(a, off, bin + 1));
+  if (a.c.pattern) {
+    const float2 p = __ldg(reinterpret_cast<const float2*>((MODE >= 2 ? a.t.pattern3d : a.t.pattern2d) + bin));
+    return pk2(-p.x, -p.y);
+  }
+  return dup2(-a.c.sigma2n);
+}
+// Two neighbouring weights of a per-bin table, or zeros where it is not used.
+__device__ __forceinline__ f2x pair_weights(const float* table, bool use, int bin) {
+  if (!use) return 0;
+  const float2 w = __ldg(reinterpret_cast<const float2*>(table + bin));
+  return pk2(w.x, w.y);
+}
+
+// One frame of one bin pair from its window's values r[LO .. HI]. Wiener and
+// sharpen-only modes.
+template <int MODE>
+__device__ __forceinline__ float4 group_filter_one(const InverseArgs& a, size_t off, int bin, const float4 (&r)[5],
+                                                   float gf) {
+  constexpr int LO = win_lo<MODE>(), HI = win_hi<MODE>();
+  if constexpr (MODE >= 2) {
+    Pair w[5];
+#pragma unroll
+    for (int k = 0; k < 5; k++) w[k] = pair_of(r[k >= LO && k <= HI ? k : LO]);
+    return bins_of(filter_pair<MODE>(w, pair_grid(a, bin), gf, pair_noise<MODE>(a, off, bin), a.c.lowlimit));
+  } else if constexpr (MODE == MODE_WIENER2D) {
+    float2 w0[5], w1[5];
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+      w0[k] = k == 2 ? make_float2(r[2].x, r[2].y) : make_float2(0.f, 0.f);
+      w1[k] = k == 2 ? make_float2(r[2].z, r[2].w) : make_float2(0.f, 0.f);
+    }
+    const float2 v0 = filter_vals<MODE>(a, w0, off, bin, gf, bin_tab<MODE>(a, bin), false);
+    const float2 v1 = filter_vals<MODE>(a, w1, off, bin + 1, gf, bin_tab<MODE>(a, bin + 1), false);
+    return make_float4(v0.x, v0.y, v1.x, v1.y);
+  } else {
+    return r[2];
+  }
+}
+
 // ---------------------------------------------------------------- filter (streaming)
 
 // Two neighbouring bins of a window spectrum, read once per thread: not kept
@@ -805,10 +1021,10 @@ __global__ void __launch_bounds__(256) k_filter_frames(InverseArgs a, const __gr
 // ---------------------------------------------------------------- inverse
 
 // One warp filters and inverse-transforms blocks_per_warp<BW>() blocks:
-//  A. every bin of a block, consecutive bins on consecutive lanes (coalesced
-//     loads of the bt spectra), through the filter and the separate
-//     sharpen/dehalo pass (whose grid fraction is the filtered DC, lane 0's
-//     first bin); results to shared memory;
+//  A. every bin of a block, consecutive bin pairs on consecutive lanes
+//     (coalesced 16-byte loads of the bt spectra), through the filter and the
+//     separate sharpen/dehalo pass (whose grid fraction is the filtered DC,
+//     lane 0's first bin); results to shared memory;
 //  B. one column per lane: inverse complex DFT along y (DC and Nyquist columns
 //     together: both are Hermitian, so their inverses are real);
 //  C. one row per lane: c2r along x, 16-byte stores of the time-domain rows.
@@ -828,17 +1044,12 @@ __device__ __forceinline__ float2 ld_stream(const float2* p) {
 // Where a CTA finds its window spectra and writes its time-domain blocks:
 // the launch arguments (one output frame per launch), or pointers picked for
 // one frame of a frame group (k_filter_inverse_frames).
-// kHoistTab: a chunk's per-bin table values are loaded before its filter
-// arithmetic (measured faster one frame per launch); the frame-group kernel
-// loads each next to its first use (faster there: fewer live registers).
 struct ArgsWin {
-  static constexpr bool kHoistTab = true;
   const InverseArgs& a;
   __device__ __forceinline__ const float2* in(int k) const { return a.in[k]; }
   __device__ __forceinline__ float* tdom() const { return a.tdom; }
 };
 struct FrameWin {
-  static constexpr bool kHoistTab = false;
   const float2* p[5];
   float* t;
   __device__ __forceinline__ const float2* in(int k) const { return p[k]; }
@@ -850,8 +1061,8 @@ struct FrameWin {
 template <int BW, int BH, int MODE, bool NEWEST_IN_S, class Win>
 __device__ __forceinline__ void filter_inverse_cta_w(const InverseArgs& a, int vcta, const Win& win) {
   constexpr int NH = BW / 2 + 1, HC = BW / 2, NBW = blocks_per_warp<BW>(), BINS = BH * NH;
-  constexpr int PER = (BINS + 31) / 32;
-  extern __shared__ float2 smem2[];
+  constexpr int PER = (BINS / 2 + 31) / 32;
+  extern __shared__ __align__(16) float2 smem2[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* S = smem2 + warp * NBW * BINS;
   const Geom& g = a.g;
@@ -862,9 +1073,9 @@ __device__ __forceinline__ void filter_inverse_cta_w(const InverseArgs& a, int v
   constexpr int LO = win_lo<MODE>(), HI = win_hi<MODE>(), NW = HI - LO + 1;
   constexpr int NG = NEWEST_IN_S ? NW - 1 : NW;  // window slots read from global memory
   constexpr int NGB = NG > 0 ? NG : 1;
-  // load-pipeline depth (chunks of 32 bins in flight): all chunks for a
-  // one-frame window, fewer as the window (and the registers per chunk) grows
-  constexpr int DW = NG <= 1 ? PER : (NG == 2 ? 10 : (NG == 3 ? 7 : (NG == 4 ? 5 : 4)));
+  // load-pipeline depth (chunks of 32 bin pairs in flight), fewer as the
+  // window (and the registers per chunk) grows
+  constexpr int DW = NG <= 1 ? 4 : (NG == 2 ? 4 : (NG == 3 ? 3 : 2));
   constexpr int D = PER < DW ? PER : DW;
 #pragma unroll 1
   for (int b = 0; b < NBW; b++) {
@@ -882,49 +1093,54 @@ __device__ __forceinline__ void filter_inverse_cta_w(const InverseArgs& a, int v
     }
     // software pipeline: the window's values of chunk j + D are loaded while
     // chunk j is filtered, so D x NG loads per lane are always in flight
-    float2 buf[D][NGB];
-    auto load = [&](int j, float2(&dst)[NGB]) {
-      const int i = lane + 32 * j;
+    float4 buf[D][NGB];
+    auto load = [&](int j, float4(&dst)[NGB]) {
+      const int i = 2 * (lane + 32 * j);
 #pragma unroll
       for (int k = 0; k < NG; k++)
-        dst[k] = (i < BINS && FFT3D_IN(win.in(LO + k) != nullptr && off + i < (size_t)g.nblocks * BINS, a.err))
-                     ? ld_stream(win.in(LO + k) + off + i)
-                     : make_float2(0.f, 0.f);
+        dst[k] = (i < BINS && FFT3D_IN(win.in(LO + k) != nullptr && off + i + 1 < (size_t)g.nblocks * BINS, a.err))
+                     ? ld_stream4(win.in(LO + k) + off + i)
+                     : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     if constexpr (NG > 0) {
 #pragma unroll
       for (int j = 0; j < D; j++) load(j, buf[j]);
     }
     float gsh = 0.f;
+    // (D chunks to a turn of the loop: the whole block unrolled is four times
+    // the code, and its instruction-cache misses cost more than the loop)
+#pragma unroll 1
+    for (int j0 = 0; j0 < PER; j0 += D) {
 #pragma unroll
-    for (int j = 0; j < PER; j++) {
-      const int i = lane + 32 * j;
-      float2 w[5];
+      for (int u = 0; u < D; u++) {
+        const int j = j0 + u, i = 2 * (lane + 32 * j);
+        if (j >= PER) break;
+        const bool in = i < BINS;
+        float4 w[5];
 #pragma unroll
-      for (int k = 0; k < 5; k++) w[k] = (k >= LO && k < LO + NG) ? buf[j % D][k - LO] : make_float2(0.f, 0.f);
-      if (NEWEST_IN_S && i < BINS) w[HI] = S[b * BINS + i];
-      BinTab tb{make_float2(0.f, 0.f), 0.f, 0.f};
-      if constexpr (Win::kHoistTab) {
-        // the chunk's table values first: the filter arithmetic hides their latency
-        if (i < BINS) tb = bin_tab<MODE>(a, i);
-      } else if (MODE == MODE_WIENER2D && a.c.fuse_sharpen) {
-        if (i < BINS) tb = bin_tab<MODE>(a, i);  // the Wiener factor takes the sharpen/dehalo weights
-      } else {
-        if (i < BINS && a.c.degrid != 0.f) tb.grid = __ldg(a.t.grid + i);
-      }
-      if (NG > 0 && j + D < PER) load(j + D, buf[j % D]);
-      float2 v = make_float2(0.f, 0.f);
-      if (i < BINS) v = filter_vals<MODE>(a, w, off, i, gf, tb, true);
-      if (a.c.do_sharpen) {
-        // grid fraction of the sharpen pass: the filtered DC (lane 0, chunk 0)
-        if (j == 0) gsh = a.c.degrid * __shfl_sync(0xffffffffu, v.x, 0) / gs0;
-        if constexpr (!Win::kHoistTab) {
-          if (i < BINS && a.c.use_sharpen) tb.wsh = __ldg(a.t.wsharpen + i);
-          if (i < BINS && a.c.use_dehalo) tb.wdh = __ldg(a.t.wdehalo + i);
+        for (int k = 0; k < 5; k++) w[k] = (k >= LO && k < LO + NG) ? buf[u][k - LO] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (NEWEST_IN_S && in) w[HI] = *reinterpret_cast<const float4*>(S + b * BINS + i);
+        if (NG > 0 && j + D < PER) load(j + D, buf[u]);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (in) {
+          if constexpr (MODE == MODE_KALMAN) {
+            const float2 w0[5] = {{}, {}, {w[2].x, w[2].y}, {}, {}}, w1[5] = {{}, {}, {w[2].z, w[2].w}, {}, {}};
+            const float2 v0 = filter_vals<MODE>(a, w0, off, i, gf, BinTab{}, true);
+            const float2 v1 = filter_vals<MODE>(a, w1, off, i + 1, gf, BinTab{}, true);
+            v = make_float4(v0.x, v0.y, v1.x, v1.y);
+          } else {
+            v = group_filter_one<MODE>(a, off, i, w, gf);
+          }
         }
-        if (i < BINS) v = sharpen_bin(a, v, tb, gsh);
+        if (a.c.do_sharpen) {
+          // grid fraction of the sharpen pass: the filtered DC (lane 0, chunk 0)
+          if (j == 0) gsh = a.c.degrid * __shfl_sync(0xffffffffu, v.x, 0) / gs0;
+          if (in)
+            v = bins_of(sharpen_pair(a, pair_of(v), pair_grid(a, i), pair_weights(a.t.wsharpen, a.c.use_sharpen, i),
+                                     pair_weights(a.t.wdehalo, a.c.use_dehalo, i), gsh));
+        }
+        if (in) *reinterpret_cast<float4*>(S + b * BINS + i) = v;
       }
-      if (i < BINS) S[b * BINS + i] = v;
     }
   }
   __syncwarp();
@@ -974,7 +1190,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_filter_inverse_frames(InverseAr
 }
 
 template <int BW, int BH, int MODE>
-__global__ void __launch_bounds__(kWarps * 32) k_filter_inverse(InverseArgs a) {
+__global__ void __launch_bounds__(kWarps * 32, ctas_for(5, kWarps * fft_smem_bytes<BW, BH>())) k_filter_inverse(InverseArgs a) {
   filter_inverse_cta<BW, BH, MODE>(a, blockIdx.x);
 }
 
@@ -1208,38 +1424,52 @@ __device__ __forceinline__ void overlap_add_px4(const OlaArgs& a, int x0, int k)
   ola4_finish<T>(a, a.dst, a.dst_stride, x0, k, p);
 }
 
-// ---------------------------------------------------------------- frame groups, one CTA per block
+// ---------------------------------------------------------------- bulk copies
 
-// Dynamic shared memory of k_filter_inverse_group: two grid fractions per
-// frame (64 bytes), then `count` spectrum tiles.
-template <int BW, int BH>
-__host__ __device__ constexpr int group_smem_bytes(int count) {
-  return 2 * kGroupTile * 4 + count * BH * (BW / 2 + 1) * 8;
+constexpr int kBulkSpin = 1 << 22;  // bounded mbarrier wait (then error flag 2)
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool bulk_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t done = 0;
+  for (int it = 0; it < kBulkSpin && !done; it++)
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+  return done != 0;
 }
 
-// A run of count <= kGroupTile consecutive output frames of one plane with
-// one mode; CTA = one block. Each stage is spread over the whole CTA, with a
-// barrier between stages:
-//  0. the grid fraction of each frame's block (its DC);
-//  1. filter: each thread takes two neighbouring bins and walks the run's
-//     frames in order, its window of MODE frames in registers (a circular
-//     buffer; the next frame's bins loaded one frame ahead), so that each of
-//     the block's count + MODE - 1 window spectra is read once for the run
-//     (and a Kalman state once); the filtered bins of frame j go to tile j in
-//     shared memory, and the thread holding the DC publishes each tile's
-//     filtered DC;
-//     (pairs beyond the last whole round of the CTA's threads are spread
-//     over all threads as single (pair, frame) items, so that no warp walks
-//     a third round alone);
-//  2. the separate sharpen/dehalo pass (src/code_impl/Sharpen.cpp:13-63), its
-//     grid fraction from each tile's filtered DC, the pair's tables loaded
-//     once for all frames;
-//  3. the inverse column DFTs of every tile (DC and Nyquist columns as one
-//     complex transform), 4. the c2r rows, 5. coalesced stores of the
-//     time-domain blocks.
-// Every bin and every transform uses the arithmetic of k_filter_inverse
-// (filter_vals, kalman_step, sharpen_bin, inv_col, inv_row_inplace), so the
-// output equals one frame per launch.
+// One mbarrier for one arrival, made ready for the CTA's bulk copies.
+__device__ __forceinline__ void bulk_init(uint64_t* bar) {
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(1));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------- runs of frames, a few blocks per CTA
+
+// Spectrum tiles one CTA of k_filter_inverse_group works on (blocks x frames
+// of the run): as many as its 128 threads have columns for in one round of
+// the column transforms, while 6 CTAs stay resident per SM (36 KB of tiles),
+// and at least the longest run's frames.
+template <int BW, int BH>
+__host__ __device__ constexpr int group_tiles() {
+  const int lanes = kWarps * 32 / (BW / 2), fit = 36 * 1024 / (BH * (BW / 2 + 1) * 8);
+  const int t = lanes < fit ? lanes : fit, run = group_run_frames(BW, BH);
+  return t > run ? t : run;
+}
+// Two grid fractions per tile, in front of the tiles (16-byte aligned).
+template <int BW, int BH>
+__host__ __device__ constexpr int group_head_floats() { return (2 * group_tiles<BW, BH>() + 3) / 4 * 4; }
+// Dynamic shared memory of k_filter_inverse_group.
+template <int BW, int BH>
+__host__ __device__ constexpr int group_smem_bytes(int tiles) {
+  return group_head_floats<BW, BH>() * 4 + tiles * BH * (BW / 2 + 1) * 8;
+}
+
 // A run's window spectrum s, bins bin and bin + 1 of the block at `off`
 // (checked build: the spectrum exists and the pair lies in the plane).
 __device__ __forceinline__ float4 group_load(const InverseArgs& a, const TemporalSet& ts, int s, size_t off, int bin) {
@@ -1250,15 +1480,15 @@ __device__ __forceinline__ float4 group_load(const InverseArgs& a, const Tempora
   return ld_stream4(ts.spec[s] + off + bin);
 }
 
-template <int MODE>
-__device__ __forceinline__ void group_filter_pair(const InverseArgs& a, const TemporalSet& ts, size_t off, int bin,
-                                                  int count, const float* gfs, float* gsh, float gs0, float2* tile,
-                                                  int tile_stride) {
-  constexpr int LO = win_lo<MODE>(), HI = win_hi<MODE>(), NW = HI - LO + 1;
-  auto out = [&](int j, float2 v0, float2 v1) {
-    *reinterpret_cast<float4*>(tile + j * tile_stride) = make_float4(v0.x, v0.y, v1.x, v1.y);
-    if (bin == 0) gsh[j] = a.c.degrid * v0.x / gs0;  // the sharpen pass's grid fraction: the filtered DC
-  };
+// Bins bin, bin + 1 of the block at `off` through all the run's frames, in
+// order: Wiener 3D with the window of MODE frames in registers (each spectrum
+// read once, the next frame's bins loaded one frame ahead), or Kalman with
+// the state in registers. load(s): the pair in the run's window spectrum s;
+// gfs: the grid fraction of the block's first frame, tile: the pair's place in
+// its tile; both `stride` tiles apart from frame to frame.
+template <int MODE, int BINS, class Load>
+__device__ __forceinline__ void group_filter_pair(const InverseArgs& a, size_t off, int bin, int count,
+                                                  const float* gfs, float2* tile, int stride, const Load& load) {
   if constexpr (MODE == MODE_KALMAN) {
     float4 lv;
     float2 cv, cp;
@@ -1268,84 +1498,51 @@ __device__ __forceinline__ void group_filter_pair(const InverseArgs& a, const Te
     asm("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(cp.x), "=f"(cp.y) : "l"(a.kal_covarp + off + bin));
     float2 l0 = make_float2(lv.x, lv.y), l1 = make_float2(lv.z, lv.w);
     float s0 = a.c.sigma2n_2d, s1 = a.c.sigma2n_2d;
-    if (a.c.pattern) {
+    if (a.psd) {
+      s0 = fmaxf(learned_noise(a, off, bin), 1e-15f);
+      s1 = fmaxf(learned_noise(a, off, bin + 1), 1e-15f);
+    } else if (a.c.pattern) {
       s0 = fmaxf(__ldg(a.t.pattern2d + bin), 1e-15f);
       s1 = fmaxf(__ldg(a.t.pattern2d + bin + 1), 1e-15f);
     }
-    float4 nxt = group_load(a, ts, 2, off, bin);
+    float4 nxt = load(2);
     for (int j = 0; j < count; j++) {
       const float4 c = nxt;
-      if (j + 1 < count) nxt = group_load(a, ts, j + 3, off, bin);
+      if (j + 1 < count) nxt = load(j + 3);
       kalman_step(a, make_float2(c.x, c.y), s0, l0, cv.x, cp.x);
       kalman_step(a, make_float2(c.z, c.w), s1, l1, cv.y, cp.y);
-      out(j, l0, l1);
+      *reinterpret_cast<float4*>(tile + j * stride * BINS) = make_float4(l0.x, l0.y, l1.x, l1.y);
     }
     *reinterpret_cast<float4*>(a.kal_last + off + bin) = make_float4(l0.x, l0.y, l1.x, l1.y);
     *reinterpret_cast<float2*>(a.kal_covar + off + bin) = cv;
     *reinterpret_cast<float2*>(a.kal_covarp + off + bin) = cp;
-  } else if constexpr (MODE == MODE_SHARPEN_ONLY) {
-    for (int j = 0; j < count; j++) {
-      const float4 c = group_load(a, ts, j + 2, off, bin);
-      out(j, make_float2(c.x, c.y), make_float2(c.z, c.w));
-    }
-  } else {
-    const BinTab tb0 = bin_tab<MODE>(a, bin), tb1 = bin_tab<MODE>(a, bin + 1);
+  } else if constexpr (MODE >= 2) {
+    constexpr int LO = win_lo<MODE>(), HI = win_hi<MODE>(), NW = HI - LO + 1;
+    const Pair grid = pair_grid(a, bin);
+    const f2x nn = pair_noise<MODE>(a, off, bin);
     // spectrum s (frame n0 - 2 + s) lives in r[s % NW]; frame j reads
     // s = j + LO .. j + HI; with j = j0 + u and j0 a multiple of NW every
     // index below is a compile-time constant
-    float4 r[NW];
+    Pair r[NW];
 #pragma unroll
-    for (int k = 0; k < NW - 1; k++) r[(LO + k) % NW] = group_load(a, ts, LO + k, off, bin);
-    float4 nxt = group_load(a, ts, HI, off, bin);
-    for (int j0 = 0; j0 < count; j0 += NW) {
+    for (int k = 0; k < NW - 1; k++) r[(LO + k) % NW] = pair_of(load(LO + k));
+    float4 nxt = load(HI);
+    // (left by a return from inside the unrolled steps: with a condition around
+    // each step the window's registers are moved at every join)
+    for (int j = 0;;) {
 #pragma unroll
       for (int u = 0; u < NW; u++) {
-        const int j = j0 + u;
-        if (j < count) {
-          r[(u + HI) % NW] = nxt;
-          if (j + 1 < count) nxt = group_load(a, ts, j + 1 + HI, off, bin);
-          float2 w0[5], w1[5];
+        r[(u + HI) % NW] = pair_of(nxt);
+        if (j + 1 < count) nxt = load(j + 1 + HI);
+        Pair w[5];
 #pragma unroll
-          for (int k = 0; k < 5; k++) {
-            const bool in = k >= LO && k <= HI;
-            const float4 v = r[(u + (in ? k : LO)) % NW];
-            w0[k] = in ? make_float2(v.x, v.y) : make_float2(0.f, 0.f);
-            w1[k] = in ? make_float2(v.z, v.w) : make_float2(0.f, 0.f);
-          }
-          const float gf = gfs[j];
-          out(j, filter_vals<MODE>(a, w0, off, bin, gf, tb0, false), filter_vals<MODE>(a, w1, off, bin + 1, gf, tb1, false));
-        }
+        for (int k = 0; k < 5; k++) w[k] = r[(u + (k >= LO && k <= HI ? k : LO)) % NW];
+        const Pair v = filter_pair<MODE>(w, grid, gfs[j * stride], nn, a.c.lowlimit);
+        *reinterpret_cast<float4*>(tile + j * stride * BINS) = bins_of(v);
+        if (++j == count) return;
       }
     }
   }
-}
-
-// One frame of one bin pair (the tail of the filter stage, spread over all
-// threads): the pair's window for frame j loaded directly. Wiener modes.
-template <int MODE>
-__device__ __forceinline__ void group_filter_one(const InverseArgs& a, const TemporalSet& ts, size_t off, int bin, int j,
-                                                 const float* gfs, float* gsh, float gs0, float2* tile) {
-  constexpr int LO = win_lo<MODE>(), HI = win_hi<MODE>();
-  float4 r[5];
-#pragma unroll
-  for (int k = LO; k <= HI; k++) r[k] = group_load(a, ts, j + k, off, bin);
-  float2 w0[5], w1[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    const bool in = k >= LO && k <= HI;
-    w0[k] = in ? make_float2(r[k].x, r[k].y) : make_float2(0.f, 0.f);
-    w1[k] = in ? make_float2(r[k].z, r[k].w) : make_float2(0.f, 0.f);
-  }
-  float2 v0, v1;
-  if constexpr (MODE == MODE_SHARPEN_ONLY) {
-    v0 = w0[2];
-    v1 = w1[2];
-  } else {
-    v0 = filter_vals<MODE>(a, w0, off, bin, gfs[j], bin_tab<MODE>(a, bin), false);
-    v1 = filter_vals<MODE>(a, w1, off, bin + 1, gfs[j], bin_tab<MODE>(a, bin + 1), false);
-  }
-  *reinterpret_cast<float4*>(tile) = make_float4(v0.x, v0.y, v1.x, v1.y);
-  if (bin == 0) gsh[j] = a.c.degrid * v0.x / gs0;
 }
 
 // The overlap-add of output tile (tx, ty) (OlaFuse) for the run's frames:
@@ -1388,108 +1585,244 @@ __device__ __noinline__ void group_ola_tile(const OlaFuse& of, const TemporalSet
   }
 }
 
+// A thread's walk over the bin pairs of consecutive blocks, `STEP` pairs at a
+// time: block b and first bin, kept without divisions.
+template <int BINS, int STEP>
+struct PairCursor {
+  int b, bin;
+  __device__ __forceinline__ explicit PairCursor(int pair) : b(pair / (BINS / 2)), bin(2 * (pair % (BINS / 2))) {}
+  __device__ __forceinline__ void step() {
+    b += 2 * STEP / BINS;
+    bin += 2 * STEP % BINS;
+    if (bin >= BINS) bin -= BINS, b++;
+  }
+};
+
+// Window spectra beyond the run's own frames that a staged run keeps in shared memory.
+template <int MODE>
+__host__ __device__ constexpr int win_extra() { return MODE >= 2 ? win_hi<MODE>() - win_lo<MODE>() : 0; }
+// Whether runs of this block size and mode fetch their window spectra by bulk
+// copies into their tiles: where the longest run's tiles and its window's
+// extra ones still let 4 CTAs reside per SM.
 template <int BW, int BH, int MODE>
-__device__ __forceinline__ void filter_inverse_group_cta(const InverseArgs& a, const TemporalSet& ts, int blk,
-                                                         const OlaFuse* of = nullptr) {
+__host__ __device__ constexpr bool run_staged() {
+  return ctas_for(4, group_smem_bytes<BW, BH>(group_run_frames(BW, BH) + win_extra<MODE>())) >= 4;
+}
+// Tiles of shared memory of a CTA, and the CTAs per SM its kernel is compiled for.
+template <int BW, int BH, int MODE, bool STAGED>
+__host__ __device__ constexpr int run_tiles() {
+  const int most = group_run_frames(BW, BH) + win_extra<MODE>();
+  return STAGED && most > group_tiles<BW, BH>() ? most : group_tiles<BW, BH>();
+}
+template <int BW, int BH, int MODE, bool STAGED>
+__host__ __device__ constexpr int run_ctas(int extra) {
+  return ctas_for(STAGED || MODE < 2 ? FFT3D_GROUP_CTAS : kShortCtas,
+                  group_smem_bytes<BW, BH>(run_tiles<BW, BH, MODE, STAGED>()) + extra);
+}
+
+// A run of count <= kGroupTile consecutive output frames of one plane with
+// one mode; CTA `cta` takes ts.nb consecutive blocks, so it makes count x
+// ts.nb spectrum tiles in shared memory (tile j * blocks + b: frame j of block
+// b). Each stage is spread over the whole CTA, with a barrier between stages:
+//  0. STAGED: one bulk copy per window spectrum brings its blocks into the
+//     tiles (the window's spectra beyond the run's frames into extra tiles);
+//     the filter then works in place, since frame j's window begins with the
+//     spectrum whose tile it overwrites and one thread takes a pair through
+//     all frames. Otherwise the filter reads the spectra from global memory;
+//  1. the grid fraction of each tile (its block's DC in its frame), then the
+//     filter. Wiener 3D runs of 2 frames and more, and Kalman: each thread
+//     takes two neighbouring bins and walks the run's frames in order, its
+//     window in registers, so that each of the block's count + MODE - 1
+//     window spectra is read once for the run (and a Kalman state once);
+//     pairs beyond the last whole round of the CTA's threads, and all pairs
+//     of shorter or window-less runs, are spread over all threads as single
+//     (pair, frame) items. The thread that holds a tile's DC publishes the
+//     filtered DC;
+//  2. the separate sharpen/dehalo pass (src/code_impl/Sharpen.cpp:13-63), its
+//     grid fraction from each tile's filtered DC, the pair's tables loaded
+//     once for all frames;
+//  3. the inverse column DFTs of every tile (DC and Nyquist columns as one
+//     complex transform), 4. the c2r rows, 5. coalesced stores of the
+//     time-domain blocks.
+// bar: an initialised mbarrier (STAGED), whose parity is `phase`. False when
+// the bounded wait on it ran out (the whole CTA then leaves).
+template <int BW, int BH, int MODE, bool STAGED>
+__device__ __forceinline__ bool filter_inverse_group_cta(const InverseArgs& a, const TemporalSet& ts, int cta,
+                                                         uint64_t* bar, uint32_t phase, const OlaFuse* of = nullptr) {
   constexpr int NH = BW / 2 + 1, HC = BW / 2, BINS = BH * NH, PAIRS = BINS / 2, NT = kWarps * 32;
+  constexpr int LO = win_lo<MODE>(), HI = win_hi<MODE>();
   static_assert(BINS % 2 == 0, "bin pairs");
-  extern __shared__ float2 smem2[];
-  float* gfs = reinterpret_cast<float*>(smem2);  // grid fraction of each frame's block
-  float* gsh = gfs + kGroupTile;                 // ... and of its filtered block (sharpen pass)
-  float2* S = smem2 + kGroupTile;                // [count][BINS] tiles, 16-byte aligned
+  extern __shared__ __align__(16) float2 smem2[];
+  float* gfs = reinterpret_cast<float*>(smem2);  // grid fraction of each tile's block
+  float* gsh = gfs + group_tiles<BW, BH>();      // ... and of its filtered block (sharpen pass)
+  float2* S = smem2 + group_head_floats<BW, BH>() / 2;  // [tile][BINS], 16-byte aligned
   const int count = ts.count;
-  const size_t off = (size_t)blk * BINS;
+  const int blk0 = cta * ts.nb, nbv = min(ts.nb, a.g.nblocks - blk0);
+  if (nbv <= 0) return true;
+  const int tiles = nbv * count, npairs = nbv * PAIRS;
+  const size_t off0 = (size_t)blk0 * BINS;
   const float gs0 = __ldg(&a.t.grid[0].x);
   const int t = threadIdx.x;
-  // 0. grid fraction of each frame's block (its DC)
-  if (MODE >= 1 && t < count)
-    gfs[t] = FFT3D_IN(ts.spec[t + 2] != nullptr && blk < a.g.nblocks, a.err)
-                 ? a.c.degrid * __ldg(&ts.spec[t + 2][off].x) / gs0 : 0.f;
-  __syncthreads();
-  // 1. filter: whole rounds of bin pairs over all frames; the remaining pairs
-  //    (a partial round) as (pair, frame) items spread over every thread,
-  //    except for Kalman, whose frames follow one another
-  constexpr int FULL = (PAIRS / NT) * NT;
-  for (int p = t; p < FULL; p += NT)
-    group_filter_pair<MODE>(a, ts, off, 2 * p, count, gfs, gsh, gs0, S + 2 * p, BINS);
-  if constexpr (MODE == MODE_KALMAN) {
-    for (int p = FULL + t; p < PAIRS; p += NT)
-      group_filter_pair<MODE>(a, ts, off, 2 * p, count, gfs, gsh, gs0, S + 2 * p, BINS);
+  bool landed = true;
+  if constexpr (STAGED) {
+    const int slots = count + win_extra<MODE>();
+    const uint32_t bytes = (uint32_t)nbv * BINS * 8;
+    auto there = [&](int k) { return FFT3D_IN(ts.spec[LO + k] != nullptr && blk0 + nbv <= a.g.nblocks, a.err); };
+    if (t == 0) {
+      uint32_t total = 0;
+      for (int k = 0; k < slots; k++) total += there(k) ? bytes : 0;
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(total) : "memory");
+      for (int k = 0; k < slots; k++)
+        if (there(k))
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                  smem_addr(S + k * nbv * BINS)),
+              "l"(ts.spec[LO + k] + off0), "r"(bytes), "r"(smem_addr(bar))
+              : "memory");
+    }
+    landed = bulk_wait(bar, phase);
+  }
+  auto load = [&](int s, int b, int bin) {
+    if constexpr (STAGED) return *reinterpret_cast<const float4*>(S + ((s - LO) * nbv + b) * BINS + bin);
+    else return group_load(a, ts, s, off0 + b * BINS, bin);
+  };
+  // 1. grid fraction of each tile, and the pairs left after the whole rounds
+  //    of a walk (read here, before any tile is overwritten)
+  if (MODE >= 1 && t < tiles && landed) {
+    const int j = div_small(t, nbv), b = t - j * nbv;
+    float dc = 0.f;
+    if constexpr (STAGED) dc = S[((j + 2 - LO) * nbv + b) * BINS].x;
+    else if (FFT3D_IN(ts.spec[j + 2] != nullptr && blk0 + b < a.g.nblocks, a.err)) dc = __ldg(&ts.spec[j + 2][off0 + b * BINS].x);
+    gfs[t] = a.c.degrid * dc / gs0;
+  }
+  constexpr bool WALK = MODE == MODE_KALMAN || MODE >= 2;
+  const bool walk = MODE == MODE_KALMAN || (MODE >= 2 && count > 1);
+  int full = walk ? npairs : 0;
+  if (MODE >= 2 && walk && (npairs % NT) * count <= NT) full = npairs / NT * NT;
+  float4 r[5];
+  int rj = 0, rp = 0;  // this thread's item of the rest: frame, pair
+  bool item = false;
+  if constexpr (MODE >= 2) {
+    const int rest = npairs - full;
+    if (walk && t < rest * count) {
+      rj = div_small(t, rest);
+      rp = full + t - rj * rest;
+      item = true;
+      const int b = rp / PAIRS, bin = 2 * (rp - b * PAIRS);
+#pragma unroll
+      for (int k = LO; k <= HI; k++) r[k] = load(rj + k, b, bin);
+    }
+  }
+  if constexpr (STAGED) {
+    if (__syncthreads_or(landed ? 0 : 1)) {
+      // the copies never completed: flag it, give them one more bounded wait
+      // (they target this CTA's shared memory), and stop
+      if (t == 0 && a.err) atomicOr(a.err, 2);
+      bulk_wait(bar, phase);
+      return false;
+    }
   } else {
-    for (int i = t; i < (PAIRS - FULL) * count; i += NT) {
-      const int q = div_small(i, count), j = i - q * count, p = FULL + q;
-      group_filter_one<MODE>(a, ts, off, 2 * p, j, gfs, gsh, gs0, S + j * BINS + 2 * p);
+    __syncthreads();
+  }
+  auto put = [&](int tile, int bin, const float4& v) {
+    *reinterpret_cast<float4*>(S + tile * BINS + bin) = v;
+    if (a.c.do_sharpen && bin == 0) gsh[tile] = a.c.degrid * v.x / gs0;  // the sharpen pass's grid fraction
+  };
+  if constexpr (MODE >= 2) {
+    if (item) {
+      const int b = rp / PAIRS, bin = 2 * (rp - b * PAIRS), tile = rj * nbv + b;
+      put(tile, bin, group_filter_one<MODE>(a, off0 + b * BINS, bin, r, gfs[tile]));
+    }
+  }
+  using Cursor = PairCursor<BINS, NT>;
+  if constexpr (WALK) {
+    Cursor c(t);
+    for (int q = t; q < full; q += NT, c.step()) {
+      const int b = c.b, bin = c.bin;
+      group_filter_pair<MODE, BINS>(a, off0 + b * BINS, bin, count, gfs + b, S + 2 * q, nbv,
+                                    [&](int s) { return load(s, b, bin); });
+      if (a.c.do_sharpen && bin == 0)
+        for (int j = 0; j < count; j++) gsh[j * nbv + b] = a.c.degrid * S[(j * nbv + b) * BINS].x / gs0;
+    }
+  }
+  if (!walk) {  // single (pair, frame) items, tile after tile, the next one's window loaded ahead
+    if constexpr (MODE != MODE_KALMAN) {
+      // (c.b counts tiles: frame cj, block c.b - cj * nbv)
+      Cursor c(t);
+      int cj = 0;
+      while (c.b >= (cj + 1) * nbv) cj++;
+      float4 nx[5];
+      auto fetch = [&]() {
+#pragma unroll
+        for (int k = LO; k <= HI; k++) nx[k] = load(cj + k, c.b - cj * nbv, c.bin);
+      };
+      const int total = tiles * PAIRS;
+      if (t < total) fetch();
+      for (int q = t; q < total; q += NT) {
+        const int tile = c.b, bin = c.bin, b = tile - cj * nbv;
+#pragma unroll
+        for (int k = LO; k <= HI; k++) r[k] = nx[k];
+        c.step();
+        while (c.b >= (cj + 1) * nbv) cj++;
+        if (q + NT < total) fetch();
+        put(tile, bin, group_filter_one<MODE>(a, off0 + b * BINS, bin, r, MODE >= 1 ? gfs[tile] : 0.f));
+      }
     }
   }
   __syncthreads();
-  // 2. the separate sharpen/dehalo pass (src/code_impl/Sharpen.cpp:13-63),
-  //    its grid fraction from each tile's filtered DC (published by the
-  //    filter stage); whole rounds of bin pairs with the pair's tables loaded
-  //    once for all frames, then the remaining pairs as (pair, frame) items
-  //    spread over every thread (as the filter stage does)
+  // 2. sharpen/dehalo: whole rounds of bin pairs with the pair's tables
+  //    loaded once for all frames, then the remaining pairs as (pair, frame)
+  //    items
   if (a.c.do_sharpen) {
-    auto tabs = [&](int bin, BinTab& tb0, BinTab& tb1) {
-      tb0 = BinTab{make_float2(0.f, 0.f), 0.f, 0.f};
-      tb1 = tb0;
-      if (a.c.degrid != 0.f) {
-        const float4 g = __ldg(reinterpret_cast<const float4*>(a.t.grid + bin));
-        tb0.grid = make_float2(g.x, g.y);
-        tb1.grid = make_float2(g.z, g.w);
-      }
-      if (a.c.use_sharpen) {
-        tb0.wsh = __ldg(a.t.wsharpen + bin);
-        tb1.wsh = __ldg(a.t.wsharpen + bin + 1);
-      }
-      if (a.c.use_dehalo) {
-        tb0.wdh = __ldg(a.t.wdehalo + bin);
-        tb1.wdh = __ldg(a.t.wdehalo + bin + 1);
-      }
+    auto one = [&](float2* at, const Pair& grid, f2x wsh, f2x wdh, float gf) {
+      float4* q = reinterpret_cast<float4*>(at);
+      *q = bins_of(sharpen_pair(a, pair_of(*q), grid, wsh, wdh, gf));
     };
-    auto one = [&](int bin, int j, const BinTab& tb0, const BinTab& tb1) {
-      float4* q = reinterpret_cast<float4*>(S + j * BINS + bin);
-      const float4 v = *q;
-      const float2 v0 = sharpen_bin(a, make_float2(v.x, v.y), tb0, gsh[j]);
-      const float2 v1 = sharpen_bin(a, make_float2(v.z, v.w), tb1, gsh[j]);
-      *q = make_float4(v0.x, v0.y, v1.x, v1.y);
-    };
-    for (int p = t; p < FULL; p += NT) {
-      BinTab tb0, tb1;
-      tabs(2 * p, tb0, tb1);
-      for (int j = 0; j < count; j++) one(2 * p, j, tb0, tb1);
+    const int whole = npairs * count <= NT ? 0 : npairs / NT * NT, rest = npairs - whole;
+    Cursor c(t);
+    for (int q = t; q < whole; q += NT, c.step()) {
+      const Pair grid = pair_grid(a, c.bin);
+      const f2x wsh = pair_weights(a.t.wsharpen, a.c.use_sharpen, c.bin),
+                wdh = pair_weights(a.t.wdehalo, a.c.use_dehalo, c.bin);
+      for (int j = 0; j < count; j++) one(S + j * nbv * BINS + 2 * q, grid, wsh, wdh, gsh[j * nbv + c.b]);
     }
-    for (int i = t; i < (PAIRS - FULL) * count; i += NT) {
-      const int q = div_small(i, count), j = i - q * count;
-      BinTab tb0, tb1;
-      tabs(2 * (FULL + q), tb0, tb1);
-      one(2 * (FULL + q), j, tb0, tb1);
+    for (int i = t; i < rest * count; i += NT) {
+      const int j = div_small(i, rest), p = whole + i - j * rest, b = p / PAIRS, bin = 2 * (p - b * PAIRS);
+      one(S + j * nbv * BINS + 2 * p, pair_grid(a, bin), pair_weights(a.t.wsharpen, a.c.use_sharpen, bin),
+          pair_weights(a.t.wdehalo, a.c.use_dehalo, bin), gsh[j * nbv + b]);
     }
     __syncthreads();
   }
   // 3. inverse column DFTs
-  for (int i = t; i < count * HC; i += NT) {
-    const int j = i / HC;
-    inv_col<BW, BH>(S + j * BINS, i - j * HC);
+  for (int i = t; i < tiles * HC; i += NT) {
+    const int k = i / HC;
+    inv_col<BW, BH>(S + k * BINS, i - k * HC);
   }
   __syncthreads();
   // 4. c2r rows, in place
-  for (int i = t; i < count * BH; i += NT) {
-    const int j = i / BH;
-    inv_row_inplace<BW, BH>(S + j * BINS, i - j * BH);
+  for (int i = t; i < tiles * BH; i += NT) {
+    const int k = i / BH;
+    inv_row_inplace<BW, BH>(S + k * BINS, i - k * BH);
   }
   __syncthreads();
   // 5. time-domain blocks (rows of BW floats, left in the tiles with a pitch of NH complex)
   constexpr int HALF = BW / 2;
-  for (int i = t; i < count * BH * HALF; i += NT) {
-    const int j = i / (BH * HALF), r = i - j * (BH * HALF);
-    const int y = r / HALF, x = r - y * HALF;
-    if (FFT3D_IN(ts.tdom[j] != nullptr && blk < a.g.nblocks, a.err))
-      reinterpret_cast<float2*>(ts.tdom[j] + (size_t)blk * BH * BW)[r] = S[j * BINS + y * NH + x];
-  }
-  // 6. the overlap-adds of the output tiles whose last block this is (OlaFuse):
-  //    release (a barrier after the stores, then a fence before each tile
-  //    arrival), acquire (a fence after the arrival that completes a tile,
-  //    then a barrier); no waiting
+  for (int j = 0, k = 0; j < count; j++)
+    for (int b = 0; b < nbv; b++, k++) {
+      float2* o = reinterpret_cast<float2*>(ts.tdom[j] + (size_t)(blk0 + b) * BH * BW);
+      if (!FFT3D_IN(ts.tdom[j] != nullptr && blk0 + b < a.g.nblocks, a.err)) continue;
+      for (int r = t; r < BH * HALF; r += NT) {
+        const int y = r / HALF, x = r - y * HALF;
+        o[r] = S[k * BINS + y * NH + x];
+      }
+    }
+  // 6. the overlap-adds of the output tiles whose last block this is (OlaFuse,
+  //    one block per CTA): release (a barrier after the stores, then a fence
+  //    before each tile arrival), acquire (a fence after the arrival that
+  //    completes a tile, then a barrier); no waiting
   if (of) {
+    const int blk = blk0;
     __shared__ int done[4];
     __syncthreads();  // the CTA's stores precede the arrivals below (the fence there is cumulative)
     const int bx = blk % a.g.nox, by = blk / a.g.nox;
@@ -1514,31 +1847,33 @@ __device__ __forceinline__ void filter_inverse_group_cta(const InverseArgs& a, c
       else group_ola_tile<float>(*of, ts, count, tx, ty);
     }
   }
+  return true;
 }
 
-template <int BW, int BH, int MODE>
-__global__ void __launch_bounds__(kWarps * 32,
-                                  ctas_for(FFT3D_GROUP_CTAS, group_smem_bytes<BW, BH>(group_run_frames(BW, BH))))
-    k_filter_inverse_group(InverseArgs a,
-                                                                     const __grid_constant__ TemporalSet ts,
-                                                                     const __grid_constant__ OlaFuse of) {
-  filter_inverse_group_cta<BW, BH, MODE>(a, ts, blockIdx.x, of.cnt ? &of : nullptr);
+template <int BW, int BH, int MODE, bool STAGED>
+__global__ void __launch_bounds__(kWarps * 32, run_ctas<BW, BH, MODE, STAGED>(0))
+    k_filter_inverse_group(InverseArgs a, const __grid_constant__ TemporalSet ts, const __grid_constant__ OlaFuse of) {
+  __shared__ uint64_t bar;
+  if constexpr (STAGED) bulk_init(&bar);
+  filter_inverse_group_cta<BW, BH, MODE, STAGED>(a, ts, a.reverse ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x,
+                                                 &bar, 0, of.cnt ? &of : nullptr);
 }
 
-// Batched runs of many planes: work item (run, block of that run's plane). The
+// Batched runs of many planes: work item (run, CTA of that run). The
 // run's arguments are staged in shared memory behind the tiles, so the body's
 // stores cannot alias them (a reference into global memory would be reloaded
 // after every store) and they cost no registers.
 template <int BW, int BH, int MODE>
-__global__ void __launch_bounds__(kWarps * 32,
-                                  ctas_for(FFT3D_GROUP_CTAS,
-                                           group_smem_bytes<BW, BH>(group_run_frames(BW, BH)) + (int)sizeof(GroupRun)))
-    k_filter_inverse_group_batch(const GroupRun* __restrict__ runs,
-                                                                           const int2* __restrict__ items,
-                                                                           int nitems) {
-  extern __shared__ float2 smem2[];
-  GroupRun* sr = reinterpret_cast<GroupRun*>(smem2 + kGroupTile + group_run_frames(BW, BH) * BH * (BW / 2 + 1));
+__global__ void __launch_bounds__(kWarps * 32, run_ctas<BW, BH, MODE, run_staged<BW, BH, MODE>()>((int)sizeof(GroupRun)))
+    k_filter_inverse_group_batch(const GroupRun* __restrict__ runs, const int2* __restrict__ items, int nitems) {
+  constexpr bool STAGED = run_staged<BW, BH, MODE>();
+  extern __shared__ __align__(16) float2 smem2[];
+  __shared__ uint64_t bar;
+  GroupRun* sr = reinterpret_cast<GroupRun*>(reinterpret_cast<char*>(smem2) +
+                                             group_smem_bytes<BW, BH>(run_tiles<BW, BH, MODE, STAGED>()));
   static_assert(sizeof(GroupRun) % 4 == 0, "word copy");
+  if constexpr (STAGED) bulk_init(&bar);
+  uint32_t phase = 0;
   for (int i = blockIdx.x; i < nitems; i += gridDim.x) {
     const int2 it = items[i];
     __syncthreads();  // every thread is done with the previous item's arguments and tiles
@@ -1546,27 +1881,14 @@ __global__ void __launch_bounds__(kWarps * 32,
     int* dst = reinterpret_cast<int*>(sr);
     for (int w = threadIdx.x; w < (int)(sizeof(GroupRun) / 4); w += blockDim.x) dst[w] = src[w];
     __syncthreads();
-    filter_inverse_group_cta<BW, BH, MODE>(sr->a, sr->ts, it.y);
+    if (!filter_inverse_group_cta<BW, BH, MODE, STAGED>(sr->a, sr->ts, it.y, &bar, phase)) return;
+    phase ^= 1;
   }
 }
 
 // ---------------------------------------------------------------- inverse (bulk-staged)
 
 constexpr int kBulkWarps = 4;
-constexpr int kBulkSpin = 1 << 22;  // bounded mbarrier wait (then error flag 2)
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool bulk_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t done = 0;
-  for (int it = 0; it < kBulkSpin && !done; it++)
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-  return done != 0;
-}
-
 template <int BW, int BH, int MODE>
 __host__ __device__ constexpr int bulk_warp_bytes() {
   return (win_hi<MODE>() - win_lo<MODE>() + 2) * BH * (BW / 2 + 1) * 8;
@@ -1743,7 +2065,7 @@ int occupancy_of(int which, int mode_or_bytes) {
   if (which == 0) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_forward_batch<BW, BH, uint8_t>, kWarps * 32, smem);
   } else if (which == 3) {
-    const int gsmem = group_smem_bytes<BW, BH>(group_run_frames(BW, BH)) + (int)sizeof(GroupRun);
+    const int gsmem = group_smem_bytes<BW, BH>(run_tiles<BW, BH, 5, run_staged<BW, BH, 5>()>()) + (int)sizeof(GroupRun);
     fft3d::smem_attr(k_filter_inverse_group_batch<BW, BH, 5>, gsmem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_filter_inverse_group_batch<BW, BH, 5>, kWarps * 32, gsmem);
   } else {
@@ -1779,6 +2101,50 @@ cudaError_t fwd_sized(const ForwardArgs& a, int bytes, cudaStream_t s) {
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+// Blocks per CTA of a run whose block takes `count` tiles, over nblocks
+// blocks: as many as the CTA has tiles for, but no more than keep every CTA
+// slot of the chip filled (6 per SM), down to one block per CTA for small
+// planes.
+template <int BW, int BH, int MODE, bool STAGED>
+int group_blocks_per_cta(int nblocks, int count) {
+  const int most = std::max(1, run_tiles<BW, BH, MODE, STAGED>() / count);
+  const int slots = 148 * run_ctas<BW, BH, MODE, STAGED>(0);
+  return std::max(1, std::min(most, nblocks / slots));
+}
+
+template <int BW, int BH, int MODE, bool STAGED>
+cudaError_t inv_group_launch(const InverseArgs& a, const TemporalSet& ts, const OlaFuse& of, cudaStream_t s) {
+  cudaError_t e = fft3d::smem_attr(k_filter_inverse_group<BW, BH, MODE, STAGED>,
+                                   group_smem_bytes<BW, BH>(run_tiles<BW, BH, MODE, STAGED>()));
+  if (e != cudaSuccess) return e;
+  TemporalSet t = ts;
+  const int per = ts.count + (STAGED ? win_extra<MODE>() : 0);
+  t.nb = of.cnt ? 1 : group_blocks_per_cta<BW, BH, MODE, STAGED>(a.g.nblocks, per);
+  k_filter_inverse_group<BW, BH, MODE, STAGED><<<(a.g.nblocks + t.nb - 1) / t.nb, kWarps * 32,
+                                                 group_smem_bytes<BW, BH>(t.nb * per), s>>>(a, t, of);
+  return cudaGetLastError();
+}
+
+template <int BW, int BH, int MODE>
+cudaError_t inv_group_mode(const InverseArgs& a, const TemporalSet& ts, const OlaFuse& of, cudaStream_t s) {
+  if constexpr (run_staged<BW, BH, MODE>()) {
+    if (MODE < 2 || ts.count > 1) return inv_group_launch<BW, BH, MODE, true>(a, ts, of, s);
+  }
+  if constexpr (MODE >= 2 || !run_staged<BW, BH, MODE>()) return inv_group_launch<BW, BH, MODE, false>(a, ts, of, s);
+  return cudaErrorInvalidValue;
+}
+
+// One output frame of a Wiener 3D plane: large planes by k_filter_inverse (a
+// warp owns its blocks; no barriers, 2 x MODE loads in flight per lane), small
+// ones by k_filter_inverse_group with a CTA per block or two, which fills the
+// chip with fewer blocks and has a quarter of the serial work per thread.
+// Measured at bt = 5, 32 x 32 blocks, one stream: 8349 blocks 58 us by warps,
+// 67 us by CTAs; 2135 blocks 30 us and 27 us. Wiener 2D, Kalman and
+// sharpen-only frames read one spectrum, which a bulk copy brings in: by CTAs
+// at every size (8349 blocks at bt = 1: 43 us, 55 us by warps).
+template <int MODE>
+bool one_frame_by_warps(int nblocks) { return MODE >= 2 && nblocks > 4000; }
+
 template <int BW, int BH, int MODE>
 cudaError_t inv_mode(const InverseArgs& a, cudaStream_t s) {
   constexpr int bulk_smem = 128 + kBulkWarps * bulk_warp_bytes<BW, BH, MODE>();
@@ -1795,13 +2161,21 @@ cudaError_t inv_mode(const InverseArgs& a, cudaStream_t s) {
     k_filter_inverse_bulk<BW, BH, MODE><<<grid, kBulkWarps * 32, bulk_smem, s>>>(a);
     return cudaGetLastError();
   }
-  const int smem = kWarps * fft_smem_bytes<BW, BH>();
-  const int grid = fft_grid<BW, BH>(a.g.nblocks);
-  cudaError_t e =
-      fft3d::smem_attr(k_filter_inverse<BW, BH, MODE>, smem);
-  if (e != cudaSuccess) return e;
-  k_filter_inverse<BW, BH, MODE><<<grid, kWarps * 32, smem, s>>>(a);
-  return cudaGetLastError();
+  if constexpr (MODE >= 2) {
+    if (one_frame_by_warps<MODE>(a.g.nblocks)) {
+      const int smem = kWarps * fft_smem_bytes<BW, BH>();
+      cudaError_t e = fft3d::smem_attr(k_filter_inverse<BW, BH, MODE>, smem);
+      if (e != cudaSuccess) return e;
+      k_filter_inverse<BW, BH, MODE><<<fft_grid<BW, BH>(a.g.nblocks), kWarps * 32, smem, s>>>(a);
+      return cudaGetLastError();
+    }
+  }
+  // one frame is a run of one
+  TemporalSet ts{};
+  ts.count = 1;
+  for (int k = 0; k < 5; k++) ts.spec[k] = a.in[k];
+  ts.tdom[0] = a.tdom;
+  return inv_group_mode<BW, BH, MODE>(a, ts, OlaFuse{}, s);
 }
 
 template <int BW, int BH, typename T, int MODE>
@@ -1881,16 +2255,6 @@ cudaError_t inv_frames(const InverseArgs& a, const FrameSet& fs, int mode, cudaS
   return cudaErrorInvalidValue;
 }
 
-template <int BW, int BH, int MODE>
-cudaError_t inv_group_mode(const InverseArgs& a, const TemporalSet& ts, const OlaFuse& of, cudaStream_t s) {
-  const int smem = group_smem_bytes<BW, BH>(kGroupTile);
-  cudaError_t e = fft3d::smem_attr(k_filter_inverse_group<BW, BH, MODE>, smem);
-  if (e != cudaSuccess) return e;
-  k_filter_inverse_group<BW, BH, MODE>
-      <<<a.g.nblocks, kWarps * 32, group_smem_bytes<BW, BH>(ts.count), s>>>(a, ts, of);
-  return cudaGetLastError();
-}
-
 template <int BW, int BH>
 cudaError_t inv_group(const InverseArgs& a, const TemporalSet& ts, int mode, cudaStream_t s, const OlaFuse* ofp) {
   if (ts.count < 1 || ts.count > group_run_frames(BW, BH)) return cudaErrorInvalidValue;
@@ -1915,7 +2279,7 @@ cudaError_t inv_group(const InverseArgs& a, const TemporalSet& ts, int mode, cud
 
 template <int BW, int BH, int MODE>
 cudaError_t inv_group_batch_mode(const BatchLaunch& l, cudaStream_t s) {
-  const int smem = group_smem_bytes<BW, BH>(group_run_frames(BW, BH)) + (int)sizeof(GroupRun);
+  const int smem = group_smem_bytes<BW, BH>(run_tiles<BW, BH, MODE, run_staged<BW, BH, MODE>()>()) + (int)sizeof(GroupRun);
   cudaError_t e = fft3d::smem_attr(k_filter_inverse_group_batch<BW, BH, MODE>, smem);
   if (e != cudaSuccess) return e;
   k_filter_inverse_group_batch<BW, BH, MODE><<<l.grid, kWarps * 32, smem, s>>>(static_cast<const GroupRun*>(l.args),
