@@ -552,11 +552,35 @@ int spectrum_slot(fft3d_plane* P, int m, int lo, int hi, const void* plane, int 
   return FFT3D_OK;
 }
 
+// The plane's interior, which the overlap-add writes, for the crop borders'
+// copy (its frames are filled in by the caller).
+fft3d::BorderSet border_set(const fft3d_plane* P) {
+  fft3d::BorderSet b{};
+  b.width = P->d.width * P->bytes;
+  b.height = P->d.height;
+  b.x0 = P->l * P->bytes;
+  b.x1 = (P->l + P->g.W) * P->bytes;
+  b.y0 = P->t;
+  b.y1 = P->t + P->g.H;
+  return b;
+}
+
 int copy_plane(fft3d_plane* P, void* dst, int dstride, const void* src, int sstride, cudaMemcpyKind kind,
-               cudaStream_t st) {
+               cudaStream_t st, bool borders = false) {
   if (g_defer && kind == cudaMemcpyDeviceToDevice) {
     g_defer->copies.push_back({dst, (size_t)dstride, src, (size_t)sstride, (size_t)P->d.width * P->bytes,
-                               (size_t)P->d.height, g_defer->plane});
+                               (size_t)P->d.height, g_defer->plane, borders});
+    return FFT3D_OK;
+  }
+  if (borders && kind == cudaMemcpyDeviceToDevice) {
+    fft3d::BorderSet b = border_set(P);
+    b.src[0] = src;
+    b.dst[0] = dst;
+    b.spitch[0] = sstride;
+    b.dpitch[0] = dstride;
+    b.count = 1;
+    CK(fft3d::launch_copy_borders(b, st), "crop borders");
+    g_launches++;
     return FFT3D_OK;
   }
   CK(cudaMemcpy2DAsync(dst, dstride, src, sstride, (size_t)P->d.width * P->bytes, P->d.height, kind, st),
@@ -587,7 +611,7 @@ int output_frame(fft3d_plane* P, float* tdom, const fft3d::Tables& tab, float ba
     }
   } else if (crop) {
     if (!cur) return fail(FFT3D_E_FRAME, "neo_fft3d: the current frame is needed for the crop borders");
-    int rc = copy_plane(P, dst, dst_stride, cur, cur_stride, cudaMemcpyDeviceToDevice, st);
+    int rc = copy_plane(P, dst, dst_stride, cur, cur_stride, cudaMemcpyDeviceToDevice, st, true);
     if (rc) return rc;
   }
   fft3d::OlaArgs oa;
@@ -1112,9 +1136,27 @@ int run_group(fft3d_plane* P, const fft3d::Deferred& d, cudaStream_t st) {
   // the plane copies (a cropped frame's source plane, whose interior the
   // overlap-add then overwrites; Kalman frame 0): before any overlap-add,
   // which a run's filter/inverse launch may do itself
-  for (const auto& c : d.copies)
-    CK(cudaMemcpy2DAsync(c.dst, c.dpitch, c.src, c.spitch, c.width, c.height, cudaMemcpyDeviceToDevice, st),
-       "plane copy");
+  fft3d::BorderSet bs = border_set(P);
+  for (const auto& c : d.copies) {
+    if (!c.borders) {
+      CK(cudaMemcpy2DAsync(c.dst, c.dpitch, c.src, c.spitch, c.width, c.height, cudaMemcpyDeviceToDevice, st),
+         "plane copy");
+      continue;
+    }
+    bs.src[bs.count] = c.src;
+    bs.dst[bs.count] = c.dst;
+    bs.spitch[bs.count] = (long long)c.spitch;
+    bs.dpitch[bs.count] = (long long)c.dpitch;
+    if (++bs.count == fft3d::kMaxGroupFrames) {
+      CK(fft3d::launch_copy_borders(bs, st), "crop borders");
+      bs.count = 0;
+      g_launches++;
+    }
+  }
+  if (bs.count > 0) {
+    CK(fft3d::launch_copy_borders(bs, st), "crop borders");
+    g_launches++;
+  }
   std::vector<char> ola_done(d.ola.size(), 0);  // overlap-adds done by a run's launch
   for (size_t i = 0; P->group_split == 2 && i < d.inv.size();) {
     // One launch per run of up to group_run_frames consecutive frames of one mode,
@@ -1223,32 +1265,22 @@ int run_group(fft3d_plane* P, const fft3d::Deferred& d, cudaStream_t st) {
     g_launches++;
     i = e;
   }
-  // the other overlap-adds: one launch for all frames where the 4-pixel kernel applies
-  std::vector<const fft3d::Deferred::Ola*> rest;
-  for (size_t k = 0; k < d.ola.size(); k++)
-    if (!ola_done[k]) rest.push_back(&d.ola[k]);
-  bool merged = false;
-  if (rest.size() > 1 && rest.size() <= (size_t)fft3d::kMaxGroupFrames) {
-    fft3d::OlaFrameSet fs{};
-    fs.count = (int)rest.size();
-    for (size_t k = 0; k < rest.size(); k++) {
-      fs.tdom[k] = rest[k]->a.tdom;
-      fs.dst[k] = rest[k]->a.dst;
-      fs.dst_stride[k] = rest[k]->a.dst_stride;
-    }
-    if (fft3d::overlap_add_frames_supported(rest[0]->a, fs, rest[0]->bytes)) {
-      TimeScope ts(P, K_OLA, (double)rest.size() * (T + pix), st);
-      CK(fft3d::launch_overlap_add_frames(rest[0]->a, fs, rest[0]->bytes, st), "overlap-add kernel (frame group)");
-      merged = true;
-      g_launches++;
-    }
+  // the other overlap-adds: one launch for all frames
+  fft3d::OlaFrameSet rest{};
+  const fft3d::Deferred::Ola* first = nullptr;
+  for (size_t k = 0; k < d.ola.size(); k++) {
+    if (ola_done[k]) continue;
+    if (!first) first = &d.ola[k];
+    rest.tdom[rest.count] = d.ola[k].a.tdom;
+    rest.dst[rest.count] = d.ola[k].a.dst;
+    rest.dst_stride[rest.count] = d.ola[k].a.dst_stride;
+    rest.count++;  // at most FFT3D_MAX_FRAME_GROUP = kMaxGroupFrames records
   }
-  if (!merged)
-    for (const auto* o : rest) {
-      TimeScope ts(P, K_OLA, T + pix, st);
-      CK(fft3d::launch_overlap_add(o->a, o->bytes, st), "overlap-add kernel");
-      g_launches++;
-    }
+  if (first) {
+    TimeScope ts(P, K_OLA, rest.count * (T + pix), st);
+    CK(fft3d::launch_overlap_add_frames(first->a, rest, first->bytes, st), "overlap-add kernel (frame group)");
+    g_launches++;
+  }
   return FFT3D_OK;
 }
 

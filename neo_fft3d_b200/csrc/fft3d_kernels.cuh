@@ -246,6 +246,17 @@ struct CopyArgs {
   int height;
 };
 
+// The crop borders of a call's frames: planes of `width` bytes x height rows,
+// copied except for the interior of bytes [x0, x1) of rows [y0, y1).
+struct BorderSet {
+  const void* src[kMaxGroupFrames];
+  void* dst[kMaxGroupFrames];
+  long long spitch[kMaxGroupFrames], dpitch[kMaxGroupFrames];
+  int width, height;
+  int x0, x1, y0, y1;
+  int count;
+};
+
 // Host-side launchers (fft3d_kernels.cu). They return cudaGetLastError().
 cudaError_t launch_forward(const ForwardArgs& a, int bytes_per_sample, cudaStream_t s);
 cudaError_t launch_filter_inverse(const InverseArgs& a, int mode, cudaStream_t s);
@@ -263,10 +274,11 @@ cudaError_t launch_forward_frames(const ForwardArgs& a, const FwdFrameSet& fs, i
 cudaError_t launch_overlap_add(const OlaArgs& a, int bytes_per_sample, cudaStream_t s);
 // p[0 .. n) = v (stream-ordered state resets)
 cudaError_t launch_fill(float* p, float v, size_t n, cudaStream_t s);
-// fs.count overlap-adds of one plane in one launch (a holds what they share);
-// cudaErrorNotSupported when a frame's geometry or alignment rules out the
-// 4-pixel kernel (then launch them one by one).
+// fs.count overlap-adds of one plane in one launch (a holds what they share).
 cudaError_t launch_overlap_add_frames(const OlaArgs& a, const OlaFrameSet& fs, int bytes_per_sample, cudaStream_t s);
+// Crop borders of a call's frames in one launch.
+cudaError_t launch_copy_borders(const BorderSet& bs, cudaStream_t s);
+// Whether every frame of fs meets the 4-pixel form's geometry and alignment rules.
 bool overlap_add_frames_supported(const OlaArgs& a, const OlaFrameSet& fs, int bytes_per_sample);
 // Batched forms (work items as in BatchLaunch); OLA items are 32x8-pixel tiles.
 cudaError_t launch_forward_batch(int bw, int bh, const BatchLaunch& l, int bytes_per_sample, cudaStream_t s);

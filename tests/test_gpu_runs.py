@@ -79,3 +79,23 @@ def test_block_counts(gpu, w, h):
         ref = _filter(torch, a, 8, filt, [0])
         assert np.array_equal(ref, _filter(torch, a, 8, filt, [8]))
         assert np.array_equal(ref, _filter(torch, a, 8, filt, [2, 7]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits", [8, 16])
+@pytest.mark.parametrize("w,bw,ow,crop", [(118, 16, 6, {}), (118, 16, 8, {}), (120, 32, 10, {}), (120, 16, 8, {}),
+                                          (121, 16, 5, dict(l=3, t=2, r=6, b=4)), (126, 16, 8, dict(l=2, r=4, b=2)),
+                                          (130, 16, 8, dict(t=5, b=1))])
+def test_overlap_add_widths_and_borders(gpu, w, bw, ow, crop, bits):
+    """1, 2 and 4 pixels a thread in the overlap-add, few and many rows, with
+    crop borders copied from the source: against the restatement, and the
+    whole group against one-frame calls."""
+    import torch
+    a = synth.make_clip(w, 90, F, bits=bits, noise_sigma=5.0 * (1 << (bits - 8)), seed=51, planes=1)[0]
+    filt = dict(sigma=2.5, bt=3, bw=bw, bh=16, ow=ow, oh=5, **crop)
+    want = restate.filter_clip([a], bits=bits, **filt)[0]
+    ref = _filter(torch, a, bits, filt, [0])
+    d = np.abs(ref.astype(int) - want.astype(int))
+    assert (d <= 1).mean() >= 0.999 and d.max() <= 3, ((d <= 1).mean(), d.max())
+    for sizes in ([13], [4]):
+        assert np.array_equal(ref, _filter(torch, a, bits, filt, sizes)), sizes
