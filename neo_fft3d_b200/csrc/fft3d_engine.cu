@@ -866,7 +866,7 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
     CK(fft3d::psd::infer(P->psd_model, P->psd_work, ia.in[2], P->g.nblocks, P->psd_pooled != 0, P->psd_pow, P->d_psd,
                          st),
        "learned noise PSD");
-    g_launches += P->psd_pooled ? 10 : 8;  // features, 3 x (GEMM, bias/GELU), output
+    g_launches += P->psd_pooled ? 7 : 4;  // features, 3 layers (pooled: column sums and output)
     ia.psd = P->d_psd;
     ia.psd_scale = P->psd_strength * (mode >= 2 ? (float)btcur : 1.f);
     ia.psd_per_block = P->psd_pooled ? 0 : 1;

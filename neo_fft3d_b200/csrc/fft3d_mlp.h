@@ -17,9 +17,14 @@ inline bool gemm_shape_ok(long long M, long long N, long long K) {
 cudaError_t gemm_bf16(const void* A, long long sam, long long sak, const void* B, long long sbn, long long sbk,
                       float* C, long long ldc, int M, int N, int K, bool accumulate, int* err, cudaStream_t s);
 
-// Z = C + bias (per column); H = bf16(gelu(Z) or Z). Z and H may be null; Z may alias C.
-cudaError_t bias_act(const float* C, const float* bias, float* Z, void* H, long long rows, int cols, bool gelu,
-                     cudaStream_t s);
+// One layer: z = A B^T + bias (per column; A [M][K], B [N][K], K-major),
+// Z = z (row stride N) and H = bf16(gelu(z) or z); Z or H may be null.
+cudaError_t layer_bf16(const void* A, long long lda, const void* B, long long ldb, const float* bias, float* Z, void* H,
+                       int M, int N, int K, bool gelu, int* err, cudaStream_t s);
+// The model's output as noise power: out[m*cols + n] = exp(A B^T + bias + off) *
+// scale for the first `rows` rows and `cols` columns (a multiple of 4).
+cudaError_t layer_exp(const void* A, long long lda, const void* B, long long ldb, const float* bias, float off,
+                      float scale, float* out, long long rows, int cols, int M, int N, int K, int* err, cudaStream_t s);
 // dZ = dH * gelu'(Z); dZb = bf16(dZ). dZ may alias dH.
 cudaError_t gelu_back(const float* dH, const float* Z, float* dZ, void* dZb, long long n, cudaStream_t s);
 // Mean squared error of Y[:, :valid] (row stride ldy) against T (row stride

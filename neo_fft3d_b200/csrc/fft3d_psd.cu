@@ -404,26 +404,29 @@ __global__ void __launch_bounds__(256) k_gen_blocks(GenArgs a) {
 
 // model input from a plane's block spectra (blocks x 544 complex); power
 // divided by pow_scale (the square of the sample scale relative to 8 bits)
-__global__ void k_features(const float2* __restrict__ spec, __nv_bfloat16* X, long long blocks, float inv_pow) {
-  const long long n = blocks * IN;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const long long b = i / IN;
-    const int c = (int)(i - b * IN);
-    float x = 0.f;
-    if (c > 0 && c < BINS) {
-      const float2 s = spec[b * BINS + c];
-      x = (logf((s.x * s.x + s.y * s.y) * inv_pow + 1.f) - kFeatMean) * kFeatScale;
+// (8 features per thread: four 16-byte loads, one 16-byte store; one feature
+// per thread with a 64-bit division took 17 us for 1080p luma, 10.5 us now)
+__global__ void __launch_bounds__(256) k_features(const float2* __restrict__ spec, __nv_bfloat16* X, int blocks, float inv_pow) {
+  constexpr int PER = IN / 8;
+  const int n = blocks * PER;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int b = i / PER, c0 = 8 * (i - b * PER);
+    __align__(16) __nv_bfloat16 h[8];
+    if (c0 < BINS) {
+      const float4* p = reinterpret_cast<const float4*>(spec + (size_t)b * BINS + c0);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float4 v = __ldg(p + q);
+        const float x = (logf((v.x * v.x + v.y * v.y) * inv_pow + 1.f) - kFeatMean) * kFeatScale;
+        const float y = (logf((v.z * v.z + v.w * v.w) * inv_pow + 1.f) - kFeatMean) * kFeatScale;
+        h[2 * q] = __float2bfloat16_rn(c0 + q > 0 ? x : 0.f);  // the DC's feature is 0
+        h[2 * q + 1] = __float2bfloat16_rn(y);
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; q++) h[q] = __float2bfloat16_rn(0.f);
     }
-    X[i] = __float2bfloat16_rn(x);
-  }
-}
-
-__global__ void k_psd_blocks(const float* __restrict__ Y, float* out, long long blocks, float pow_scale) {
-  const long long n = blocks * BINS;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const long long b = i / BINS;
-    const int c = (int)(i - b * BINS);
-    out[i] = expf(Y[b * OUT + c] + kLogOffset) * pow_scale;
+    *reinterpret_cast<uint4*>(X + (size_t)b * IN + c0) = *reinterpret_cast<const uint4*>(h);
   }
 }
 
@@ -558,17 +561,20 @@ Work* work_alloc(long long rows, bool train) {
   return w;
 }
 
-// Y = MLP(X) for `rows` rows (X: rows x IN BF16)
-cudaError_t forward(fft3d_psd* m, Work* w, const __nv_bfloat16* X, long long rows, cudaStream_t s) {
+// The hidden layers for `rows` rows (X: rows x IN BF16) into H2; `keep`: the
+// pre-activations too, for the backward pass
+cudaError_t hidden(fft3d_psd* m, Work* w, const __nv_bfloat16* X, long long rows, bool keep, cudaStream_t s) {
   using namespace fft3d::mlp;
   const int R = (int)rows;
-  CKE(gemm_bf16(X, IN, 1, m->wb + O_W1, IN, 1, w->Z1, HID, R, HID, IN, false, m->err, s));
-  CKE(bias_act(w->Z1, m->w + O_B1, w->Z1, w->H1, rows, HID, true, s));
-  CKE(gemm_bf16(w->H1, HID, 1, m->wb + O_W2, HID, 1, w->Z2, HID, R, HID, HID, false, m->err, s));
-  CKE(bias_act(w->Z2, m->w + O_B2, w->Z2, w->H2, rows, HID, true, s));
-  CKE(gemm_bf16(w->H2, HID, 1, m->wb + O_W3, HID, 1, w->Y, OUT, R, OUT, HID, false, m->err, s));
-  CKE(bias_act(w->Y, m->w + O_B3, w->Y, nullptr, rows, OUT, false, s));
-  return cudaSuccess;
+  CKE(layer_bf16(X, IN, m->wb + O_W1, IN, m->w + O_B1, keep ? w->Z1 : nullptr, w->H1, R, HID, IN, true, m->err, s));
+  return layer_bf16(w->H1, HID, m->wb + O_W2, HID, m->w + O_B2, keep ? w->Z2 : nullptr, w->H2, R, HID, HID, true, m->err, s);
+}
+
+// Y = MLP(X)
+cudaError_t forward(fft3d_psd* m, Work* w, const __nv_bfloat16* X, long long rows, cudaStream_t s, bool keep = true) {
+  CKE(hidden(m, w, X, rows, keep, s));
+  return fft3d::mlp::layer_bf16(w->H2, HID, m->wb + O_W3, HID, m->w + O_B3, w->Y, nullptr, (int)rows, OUT, HID, false,
+                                m->err, s);
 }
 
 // gradients of the mean squared error into m->g (after forward on the same X)
@@ -747,14 +753,16 @@ cudaError_t infer(fft3d_psd* m, Work* w, const float2* spec, int nblocks, bool p
                   cudaStream_t s) {
   const long long rows = (nblocks + 127) / 128 * 128;
   if (rows > w->rows) return cudaErrorInvalidValue;
-  k_features<<<grid_for((long long)nblocks * IN), 256, 0, s>>>(spec, w->X, nblocks, 1.f / pow_scale);
+  k_features<<<grid_for((long long)nblocks * (IN / 8)), 256, 0, s>>>(spec, w->X, nblocks, 1.f / pow_scale);
   CKE(cudaGetLastError());
-  CKE(forward(m, w, w->X, rows, s));
   if (pooled) {
+    CKE(forward(m, w, w->X, rows, s, false));
     CKE(fft3d::mlp::colsum(w->Y, w->partial, w->mean, nblocks, OUT, 1.f / (float)nblocks, s));
     k_psd_pooled<<<(BINS + 255) / 256, 256, 0, s>>>(w->mean, out, pow_scale);
   } else {
-    k_psd_blocks<<<grid_for((long long)nblocks * BINS), 256, 0, s>>>(w->Y, out, nblocks, pow_scale);
+    CKE(hidden(m, w, w->X, rows, false, s));
+    CKE(fft3d::mlp::layer_exp(w->H2, HID, m->wb + O_W3, HID, m->w + O_B3, kLogOffset, pow_scale, out, nblocks, BINS,
+                              (int)rows, OUT, HID, m->err, s));
   }
   return cudaGetLastError();
 }

@@ -151,36 +151,76 @@ __global__ void __launch_bounds__(GT) k_gemm_bf16(const __nv_bfloat16* A, long l
 }
 
 // ---------------------------------------------------------------- pipelined GEMM (K-major operands)
-// C[m][n] (=|+=) sum_k A[m*lda + k] B[n*ldb + k], both operands contiguous
-// along K. 128 x BN tile per CTA (BN = 128, or 64 when N is not a multiple of
-// 128), K steps of 64 in a 3-stage shared-memory ring filled with 16-byte
-// cp.async copies: the MMAs of step k run while steps k+1 and k+2 load. The
-// K-major no-swizzle layout is padded by 16 bytes per 8-element K chunk, so
-// that the 8 threads filling one 128-byte row segment hit 8 different banks.
+__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
+__device__ __forceinline__ float gelu_grad(float x) {
+  const float cdf = 0.5f * (1.f + erff(x * 0.70710678118654752f));
+  const float pdf = 0.39894228040143268f * __expf(-0.5f * x * x);
+  return cdf + x * pdf;
+}
+
+
+// sum_k A[m*lda + k] B[n*ldb + k] through the epilogue `e`, both operands
+// contiguous along K. 128 x BN tile per CTA (BN = 160, 128 or 64, the first
+// that divides N), K steps of 64 in a 3-stage shared-memory ring filled with
+// 16-byte cp.async copies: the MMAs of step k run while steps k+1 and k+2
+// load, and two CTAs reside per SM. A row of a step is 128 bytes, stored with
+// the 128-byte swizzle (16-byte chunk c of row r at c ^ (r & 7)), which both
+// the copies and the MMA read without bank conflicts: in the unswizzled layout
+// with padded K chunks the MMA was the bottleneck (8448 x 512 x 576: 35 us,
+// tensor pipe 8 % busy; 17 us now, bias and GELU included).
 // Each stage's MMAs commit to that stage's mbarrier; a slot is refilled only
 // after its barrier completes (bounded waits; timeout -> err bit 0).
+//
+// The accumulator leaves tensor memory 32 columns at a time through shared
+// memory, so that a warp writes whole 128- or 64-byte row segments, and the
+// layer's bias and activation (or the model's output exponential) are applied
+// on the way: the element-wise passes over C cost 15 us a layer and 11 us for
+// the output.
 
 constexpr int PM = 128, PK = 64, PS = 3;
 
 template <int BN>
 struct PipeCfg {
-  static constexpr uint32_t LBO_A = (PM / 8) * 128 + 16;
-  static constexpr uint32_t LBO_B = (BN / 8) * 128 + 16;
-  static constexpr uint32_t SZ_A = 8 * LBO_A, SZ_B = 8 * LBO_B;
+  static constexpr uint32_t SZ_A = PM * PK * 2, SZ_B = BN * PK * 2;  // multiples of 1024: every tile is aligned for the swizzle
   static constexpr uint32_t STAGE = SZ_A + SZ_B;
-  static constexpr uint32_t SMEM = PS * STAGE + 64;  // + mbarriers and the TMEM address slot
+  static constexpr uint32_t SMEM = PS * STAGE + 64 + 1024;  // + mbarriers, the TMEM address slot, the base's alignment
+  static constexpr uint32_t COLS = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);  // TMEM columns (a power of two)
 };
 
+// K-major operand tile with the 128-byte swizzle: 8-row groups 1024 bytes apart
+__device__ __forceinline__ uint64_t sdesc_sw128(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
+         ((uint64_t)2 << 61);
+}
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
+// What becomes of the sums: with kind PLAIN, C = (C +) sum; with BIAS, z = sum +
+// bias[n], C = z (if C) and H = bf16(gelu(z) or z) (if H); with EXP, C =
+// exp(sum + bias[n] + off) * scale for the first `rows` rows and `cols` columns.
+enum { EPI_PLAIN, EPI_BIAS, EPI_EXP };
+struct GemmEpi {
+  int kind;
+  float* C;
+  long long ldc;
+  int accumulate;
+  const float* bias;
+  __nv_bfloat16* H;
+  long long ldh;
+  int act;
+  long long rows;
+  int cols;
+  float off, scale;
+};
+
 template <int BN>
 __global__ void __launch_bounds__(128) k_gemm_pipe(const __nv_bfloat16* __restrict__ A, long long lda,
-                                                   const __nv_bfloat16* __restrict__ B, long long ldb, float* C,
-                                                   long long ldc, int K, int accumulate, int* err) {
+                                                   const __nv_bfloat16* __restrict__ B, long long ldb, int K,
+                                                   const GemmEpi e, int* err) {
   using Cf = PipeCfg<BN>;
-  extern __shared__ __align__(1024) uint8_t sm[];
+  extern __shared__ __align__(1024) uint8_t sm_raw[];
+  uint8_t* sm = sm_raw + ((1024 - (smem_u32(sm_raw) & 1023)) & 1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + PS * Cf::STAGE);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + PS);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -188,7 +228,7 @@ __global__ void __launch_bounds__(128) k_gemm_pipe(const __nv_bfloat16* __restri
   const uint32_t sbase = smem_u32(sm);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                 "r"((uint32_t)BN));
+                 "r"(Cf::COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
@@ -206,12 +246,12 @@ __global__ void __launch_bounds__(128) k_gemm_pipe(const __nv_bfloat16* __restri
 #pragma unroll
     for (int j = 0; j < PM * 8 / 128; j++) {
       const int idx = tid + 128 * j, r = idx >> 3, c = idx & 7;
-      cp16(a + c * Cf::LBO_A + (r >> 3) * 128 + (r & 7) * 16, A + (long long)(m0 + r) * lda + k0 + c * 8);
+      cp16(a + r * 128 + ((c ^ (r & 7)) << 4), A + (long long)(m0 + r) * lda + k0 + c * 8);
     }
 #pragma unroll
     for (int j = 0; j < BN * 8 / 128; j++) {
       const int idx = tid + 128 * j, r = idx >> 3, c = idx & 7;
-      cp16(b + c * Cf::LBO_B + (r >> 3) * 128 + (r & 7) * 16, B + (long long)(n0 + r) * ldb + k0 + c * 8);
+      cp16(b + r * 128 + ((c ^ (r & 7)) << 4), B + (long long)(n0 + r) * ldb + k0 + c * 8);
     }
   };
   bool ok = true;
@@ -230,9 +270,8 @@ __global__ void __launch_bounds__(128) k_gemm_pipe(const __nv_bfloat16* __restri
       const uint32_t a = sbase + slot * Cf::STAGE, b = a + Cf::SZ_A;
       const uint32_t idesc = idesc_bf16(PM, BN);
 #pragma unroll
-      for (int ks = 0; ks < PK / 16; ks++) {
-        const uint64_t da = sdesc(a + ks * 2 * Cf::LBO_A, Cf::LBO_A, 128);
-        const uint64_t db = sdesc(b + ks * 2 * Cf::LBO_B, Cf::LBO_B, 128);
+      for (int ks = 0; ks < PK / 16; ks++) {  // 16 K values are 32 bytes of a row
+        const uint64_t da = sdesc_sw128(a + ks * 32), db = sdesc_sw128(b + ks * 32);
         const uint32_t acc = (kt > 0 || ks > 0) ? 1u : 0u;
         asm volatile(
             "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
@@ -257,10 +296,13 @@ __global__ void __launch_bounds__(128) k_gemm_pipe(const __nv_bfloat16* __restri
   if (failed && tid == 0) atomicOr(err, 1);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (!failed) {
-    float* crow = C + (long long)(m0 + warp * 32 + lane) * ldc + n0;
-    for (int half = 0; half < BN / 32; half++) {
+    // this warp's part of the (now free) ring: 32 rows of 32 floats, 144 bytes
+    // apart, or of 32 BF16, 80 bytes apart (odd multiples of 16: no conflicts)
+    uint8_t* stage = sm + warp * (32 * 144);
+    const long long row0 = m0 + warp * 32;
+    for (int part = 0; part < BN / 32; part++) {
       uint32_t r[32];
-      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + half * 32;
+      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + part * 32;
       asm volatile(
           "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
           "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -270,22 +312,68 @@ __global__ void __launch_bounds__(128) k_gemm_pipe(const __nv_bfloat16* __restri
             "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
           : "r"(taddr));
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      const int c0 = n0 + part * 32;  // this part's first column
+      float v[32];
 #pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-        float4 v = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                               __uint_as_float(r[j + 3]));
-        float4* dst = reinterpret_cast<float4*>(crow + half * 32 + j);
-        if (accumulate) {
-          const float4 o = *dst;
-          v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+      for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
+      if (e.kind != EPI_PLAIN) {
+        const float4* b4 = reinterpret_cast<const float4*>(e.bias + c0);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const float4 q = __ldg(b4 + j);
+          v[4 * j] += q.x, v[4 * j + 1] += q.y, v[4 * j + 2] += q.z, v[4 * j + 3] += q.w;
         }
-        *dst = v;
+      }
+      if (e.kind == EPI_EXP) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] = expf(v[j] + e.off) * e.scale;
+      }
+      if (e.C) {
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          *reinterpret_cast<float4*>(stage + lane * 144 + j * 16) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        __syncwarp();
+        const int c = c0 + 4 * (lane & 7);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int rr = 4 * i + (lane >> 3);
+          float4 q = *reinterpret_cast<const float4*>(stage + rr * 144 + (lane & 7) * 16);
+          if (e.kind == EPI_EXP && (row0 + rr >= e.rows || c >= e.cols)) continue;
+          float4* dst = reinterpret_cast<float4*>(e.C + (row0 + rr) * e.ldc + c);
+          if (e.accumulate) {
+            const float4 o = *dst;
+            q.x += o.x; q.y += o.y; q.z += o.z; q.w += o.w;
+          }
+          *dst = q;
+        }
+        __syncwarp();
+      }
+      if (e.H) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          uint32_t h[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const float x = v[8 * j + 2 * i], y = v[8 * j + 2 * i + 1];
+            const __nv_bfloat162 p = {__float2bfloat16_rn(e.act ? gelu(x) : x), __float2bfloat16_rn(e.act ? gelu(y) : y)};
+            h[i] = *reinterpret_cast<const uint32_t*>(&p);
+          }
+          *reinterpret_cast<uint4*>(stage + lane * 80 + j * 16) = make_uint4(h[0], h[1], h[2], h[3]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int rr = 8 * i + (lane >> 2);
+          const uint4 q = *reinterpret_cast<const uint4*>(stage + rr * 80 + (lane & 3) * 16);
+          *reinterpret_cast<uint4*>(e.H + (row0 + rr) * e.ldh + c0 + 8 * (lane & 3)) = q;
+        }
+        __syncwarp();
       }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)BN));
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cf::COLS));
 }
 
 // dst[c][r] = src[r][c] (BF16), 32 x 32 tiles through shared memory
@@ -305,24 +393,6 @@ __global__ void __launch_bounds__(256) k_transpose_bf16(const __nv_bfloat16* __r
 }
 
 // ---------------------------------------------------------------- element-wise
-
-__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float cdf = 0.5f * (1.f + erff(x * 0.70710678118654752f));
-  const float pdf = 0.39894228040143268f * __expf(-0.5f * x * x);
-  return cdf + x * pdf;
-}
-
-// Z = C + bias; store Z (pre-activation, FP32) and act(Z) as BF16
-__global__ void k_bias_act(const float* C, const float* bias, float* Z, __nv_bfloat16* H, long long rows, int cols,
-                           int act) {
-  const long long n = rows * cols;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float z = C[i] + bias[i % cols];
-    if (Z) Z[i] = z;
-    if (H) H[i] = __float2bfloat16_rn(act ? gelu(z) : z);
-  }
-}
 
 // dZ = dH * gelu'(Z) (BF16 copy for the next GEMMs, FP32 for the bias gradient)
 __global__ void k_gelu_back(const float* dH, const float* Z, float* dZ, __nv_bfloat16* dZb, long long n) {
@@ -400,26 +470,46 @@ int grid_for(long long n) {
 namespace fft3d {
 namespace mlp {
 
+namespace {
+
 template <int BN>
-cudaError_t launch_pipe(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* B, long long ldb, float* C,
-                        long long ldc, int M, int N, int K, bool accumulate, int* err, cudaStream_t s) {
+cudaError_t launch_pipe(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* B, long long ldb, int M, int N, int K,
+                        const GemmEpi& e, int* err, cudaStream_t s) {
   constexpr int smem = PipeCfg<BN>::SMEM;
-  cudaError_t e = fft3d::smem_attr(k_gemm_pipe<BN>, smem, true);
-  if (e != cudaSuccess) return e;
-  k_gemm_pipe<BN><<<dim3(N / BN, M / PM), 128, smem, s>>>(A, lda, B, ldb, C, ldc, K, accumulate ? 1 : 0, err);
+  cudaError_t rc = fft3d::smem_attr(k_gemm_pipe<BN>, smem, true);
+  if (rc != cudaSuccess) return rc;
+  k_gemm_pipe<BN><<<dim3(N / BN, M / PM), 128, smem, s>>>(A, lda, B, ldb, K, e, err);
   return cudaGetLastError();
 }
+
+// The pipelined kernel for K-major operands; the tile width is the widest that
+// divides N (160 for the model's 640 outputs: 264 CTAs for 1080p luma's 66
+// row tiles, one wave at two per SM, instead of 330).
+cudaError_t pipe_gemm(const void* A, long long lda, const void* B, long long ldb, int M, int N, int K, const GemmEpi& e,
+                      int* err, cudaStream_t s) {
+  const auto* a = static_cast<const __nv_bfloat16*>(A);
+  const auto* b = static_cast<const __nv_bfloat16*>(B);
+  if (N % 160 == 0) return launch_pipe<160>(a, lda, b, ldb, M, N, K, e, err, s);
+  if (N % 128 == 0) return launch_pipe<128>(a, lda, b, ldb, M, N, K, e, err, s);
+  return launch_pipe<64>(a, lda, b, ldb, M, N, K, e, err, s);
+}
+
+bool pipe_ok(const void* A, long long lda, const void* B, long long ldb, int M, int N, int K) {
+  return gemm_shape_ok(M, N, K) && lda % 8 == 0 && ldb % 8 == 0 && (((uintptr_t)A | (uintptr_t)B) & 15) == 0;
+}
+
+}  // namespace
 
 cudaError_t gemm_bf16(const void* A, long long sam, long long sak, const void* B, long long sbn, long long sbk,
                       float* C, long long ldc, int M, int N, int K, bool accumulate, int* err, cudaStream_t s) {
   if (!gemm_shape_ok(M, N, K)) return cudaErrorInvalidValue;
-  const bool kmajor = sak == 1 && sbk == 1 && sam % 8 == 0 && sbn % 8 == 0 &&
-                      (((uintptr_t)A | (uintptr_t)B) & 15) == 0;
-  if (kmajor) {
-    const auto* a = static_cast<const __nv_bfloat16*>(A);
-    const auto* b = static_cast<const __nv_bfloat16*>(B);
-    return N % 128 == 0 ? launch_pipe<128>(a, sam, b, sbn, C, ldc, M, N, K, accumulate, err, s)
-                        : launch_pipe<64>(a, sam, b, sbn, C, ldc, M, N, K, accumulate, err, s);
+  if (sak == 1 && sbk == 1 && pipe_ok(A, sam, B, sbn, M, N, K)) {
+    GemmEpi e{};
+    e.kind = EPI_PLAIN;
+    e.C = C;
+    e.ldc = ldc;
+    e.accumulate = accumulate ? 1 : 0;
+    return pipe_gemm(A, sam, B, sbn, M, N, K, e, err, s);
   }
   dim3 grid(N / GN, M / GM);
   k_gemm_bf16<<<grid, GT, 0, s>>>(static_cast<const __nv_bfloat16*>(A), sam, sak,
@@ -427,11 +517,33 @@ cudaError_t gemm_bf16(const void* A, long long sam, long long sak, const void* B
   return cudaGetLastError();
 }
 
-cudaError_t bias_act(const float* C, const float* bias, float* Z, void* H, long long rows, int cols, bool gelu_on,
-                     cudaStream_t s) {
-  k_bias_act<<<grid_for(rows * cols), 256, 0, s>>>(C, bias, Z, static_cast<__nv_bfloat16*>(H), rows, cols,
-                                                   gelu_on ? 1 : 0);
-  return cudaGetLastError();
+cudaError_t layer_bf16(const void* A, long long lda, const void* B, long long ldb, const float* bias, float* Z, void* H,
+                       int M, int N, int K, bool gelu_on, int* err, cudaStream_t s) {
+  if (!pipe_ok(A, lda, B, ldb, M, N, K)) return cudaErrorInvalidValue;
+  GemmEpi e{};
+  e.kind = EPI_BIAS;
+  e.C = Z;
+  e.ldc = N;
+  e.bias = bias;
+  e.H = static_cast<__nv_bfloat16*>(H);
+  e.ldh = N;
+  e.act = gelu_on ? 1 : 0;
+  return pipe_gemm(A, lda, B, ldb, M, N, K, e, err, s);
+}
+
+cudaError_t layer_exp(const void* A, long long lda, const void* B, long long ldb, const float* bias, float off,
+                      float scale, float* out, long long rows, int cols, int M, int N, int K, int* err, cudaStream_t s) {
+  if (!pipe_ok(A, lda, B, ldb, M, N, K) || cols % 4 != 0) return cudaErrorInvalidValue;
+  GemmEpi e{};
+  e.kind = EPI_EXP;
+  e.C = out;
+  e.ldc = cols;
+  e.bias = bias;
+  e.rows = rows;
+  e.cols = cols;
+  e.off = off;
+  e.scale = scale;
+  return pipe_gemm(A, lda, B, ldb, M, N, K, e, err, s);
 }
 
 cudaError_t gelu_back(const float* dH, const float* Z, float* dZ, void* dZb, long long n, cudaStream_t s) {
