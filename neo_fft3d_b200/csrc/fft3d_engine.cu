@@ -446,7 +446,10 @@ fft3d::ForwardArgs forward_args(fft3d_plane* P, const void* plane, long long str
   a.base = (P->bytes != 4 && P->d.is_chroma) ? (float)(1 << (P->d.bits - 1)) : 0.f;
   a.wan_x = P->d_wan_x;
   a.wan_y = P->d_wan_y;
-  for (int x = 0; x < fft3d::kMaxBw; x++) a.wx[x] = x < (int)P->h_wan_x.size() ? P->h_wan_x[x] : 0.f;
+  for (int x = 0; x < fft3d::kMaxBw; x++) {
+    const float w = x < (int)P->h_wan_x.size() ? 0.5f * P->h_wan_x[x] : 0.f;
+    a.wx_half[x] = make_float2(w, w);
+  }
   a.spec = spec;
   a.err = P->d_err;
   return a;
@@ -733,7 +736,7 @@ int pshow_frame(fft3d_plane* P, int n, const void* const src[5], const int strid
     if (constant) {
       a.wan_x = ones;
       a.wan_y = ones;
-      for (float& w : a.wx) w = 1.f;
+      for (float2& w : a.wx_half) w = make_float2(0.5f, 0.5f);
     }
     a.base = base;
     g_launches++;

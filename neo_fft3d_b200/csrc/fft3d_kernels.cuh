@@ -92,8 +92,8 @@ struct ForwardArgs {
   const float* wan_y;
   float2* spec;           // blocks x bh x nh
   int* err;               // device error flag (bounds-checked build), or null
-  float wx[kMaxBw];       // wan_x by value: read through the launch parameters
-                          // (constant-bank operands) by the per-plane kernels
+  float2 wx_half[kMaxBw];  // wan_x / 2 twice: pairs that the packed row transforms
+                           // read through the launch parameters (rfft_pair)
 };
 
 struct InverseArgs {

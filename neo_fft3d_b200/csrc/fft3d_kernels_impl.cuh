@@ -20,21 +20,12 @@ constexpr int kWarps = 4;       // warps per CTA in k_forward / k_filter_inverse
 // budget 65536 / (128 x CTAs): 80 registers at 6). Measured at 1080p bt=5
 // bw=32: 6 for both is 2.5 % faster than 5 (the filter/inverse spills 88
 // bytes but gains a sixth CTA).
-#ifndef FFT3D_FWD_CTAS
-#define FFT3D_FWD_CTAS 6
-#endif
 #ifndef FFT3D_GROUP_CTAS
 #define FFT3D_GROUP_CTAS 6
 #endif
 // ... and for short Wiener 3D runs, whose threads hold two windows (the one
 // they filter and the next one's loads in flight)
 constexpr int kShortCtas = 5;
-// forward rows of a lane walked by a loop (one copy of the row code) instead
-// of unrolled: fewer instruction-cache misses, the forward's largest stall
-// (measured at 1080p bw=32: 22.0 vs 23.5 us per frame over all planes)
-#ifndef FFT3D_FWD_ROW_LOOP
-#define FFT3D_FWD_ROW_LOOP 1
-#endif
 // shared memory per SM, and what the runtime reserves per resident CTA
 constexpr int kSmemPerSm = 228 * 1024, kSmemPerCtaReserved = 1024;
 __host__ __device__ constexpr int ctas_for(int want, int smem_per_cta) {
@@ -179,69 +170,28 @@ __device__ __forceinline__ const T* fwd_row_src(const ForwardArgs& a, const Win&
   return reinterpret_cast<const T*>(static_cast<const char*>(win.src()) + (long long)r * win.stride());
 }
 
-// Rows whose BW samples are whole 16-byte vectors (8- and 16-bit samples) can
-// be fetched raw ahead of their transform (forward_cta's prefetch).
-template <int BW, typename T>
-__host__ __device__ constexpr int raw_vectors() {
-  return (sizeof(T) <= 2 && (BW * (int)sizeof(T)) % 16 == 0) ? BW * (int)sizeof(T) / 16 : 0;
-}
-
-// Samples minus `base` as floats, decoded from raw 16-byte vectors. Each
-// 8/16-bit sample is placed by one byte permute into the low mantissa bits of
-// 2^23 (0x4B000000 + v is exactly the float 2^23 + v for v < 2^23), and one
-// FADD of -(2^23 + base) leaves v - base exactly: an ALU permute and an FMA-pipe
-// add per sample instead of shift/mask and an int-to-float conversion on the
-// narrower conversion pipe.
-template <int BW, typename T>
-__device__ __forceinline__ void decode_row(const uint4* raw, float base, float (&r)[BW]) {
-  constexpr int PER = 16 / (int)sizeof(T);
-  const float off = 8388608.0f + base;  // exact: base <= 2^15
-#pragma unroll
-  for (int v = 0; v < raw_vectors<BW, T>(); v++) {
-    const uint32_t w[4] = {raw[v].x, raw[v].y, raw[v].z, raw[v].w};
-#pragma unroll
-    for (int j = 0; j < PER; j++) {
-      uint32_t m;
-      if constexpr (sizeof(T) == 1) m = __byte_perm(w[j >> 2], 0x4B000000u, 0x7540u | (uint32_t)(j & 3));
-      else m = __byte_perm(w[j >> 1], 0x4B000000u, (j & 1) ? 0x7432u : 0x7410u);
-      r[v * PER + j] = __uint_as_float(m) - off;
-    }
-  }
-}
-
 // Row y of block `blk`: gather (mirrored at the plane edges), analysis window,
-// r2c along x into row y of Sb. `raw`: the row's samples already fetched
-// (interior aligned rows), or null.
-template <int BW, int BH, typename T, bool ARGS_WX, class Win>
-__device__ __forceinline__ void fwd_row(const ForwardArgs& a, const Win& win, int blk, int y, float2* Sb,
-                                        const uint4* raw) {
+// r2c along x into row y of Sb.
+template <int BW, int BH, typename T, class Win>
+__device__ __forceinline__ void fwd_row(const ForwardArgs& a, const Win& win, int blk, int y, float2* Sb) {
   constexpr int NH = BW / 2 + 1;
   const Geom& g = a.g;
   int x0, srcrow;
   const T* srow = fwd_row_src<T>(a, win, blk, y, &x0, &srcrow);
   float r[BW];
-  if constexpr (raw_vectors<BW, T>() > 0) {
-    if (raw) decode_row<BW, T>(raw, a.base, r);  // already minus base
-  }
-  if (raw_vectors<BW, T>() > 0 && raw) {
+  const bool row_ok = FFT3D_IN(srcrow >= 0 && srcrow < g.H, a.err);
+  if (x0 >= 0 && x0 + BW <= g.W) {
+    if (row_ok) load_row<T, BW>(srow + x0, r);
   } else {
-    const bool row_ok = FFT3D_IN(srcrow >= 0 && srcrow < g.H, a.err);
-    if (x0 >= 0 && x0 + BW <= g.W) {
-      if (row_ok) load_row<T, BW>(srow + x0, r);
-    } else {
 #pragma unroll
-      for (int x = 0; x < BW; x++) {
-        const int xi = reflect101(x0 + x, g.W);
-        r[x] = (row_ok && FFT3D_IN(xi >= 0 && xi < g.W, a.err)) ? load_sample<T>(srow + xi) : 0.f;
-      }
+    for (int x = 0; x < BW; x++) {
+      const int xi = reflect101(x0 + x, g.W);
+      r[x] = (row_ok && FFT3D_IN(xi >= 0 && xi < g.W, a.err)) ? load_sample<T>(srow + xi) : 0.f;
     }
-#pragma unroll
-    for (int x = 0; x < BW; x++) r[x] = r[x] - a.base;
   }
   const float wy = __ldg(a.wan_y + y);
-  // the x window from the launch parameters (ARGS_WX) or from the table
 #pragma unroll
-  for (int x = 0; x < BW; x++) r[x] = r[x] * (ARGS_WX ? a.wx[x] : __ldg(a.wan_x + x)) * wy;
+  for (int x = 0; x < BW; x++) r[x] = (r[x] - a.base) * __ldg(a.wan_x + x) * wy;
   float2 c[NH];
   rfft<BW>(r, c);
   float2* row = Sb + y * NH;
@@ -338,74 +288,22 @@ __device__ __forceinline__ void store_tdom(const float2* Sb, float* out, int lan
 
 // ---------------------------------------------------------------- forward
 
-// One warp transforms blocks_per_warp<BW>() consecutive blocks (rows, then
-// columns, then a coalesced 16-byte copy-out of the contiguous spectra).
-// PREFETCH: fetch every row of the lane before the first transform, and take
-// the x window from the launch parameters (more registers and a parameter-
-// space ForwardArgs; off where the register budget is tight or the arguments
-// are a copy in registers).
-template <int BW, int BH, typename T, bool PREFETCH, class Win>
-__device__ __forceinline__ void forward_cta_w(const ForwardArgs& a, int cta, const Win& win) {
+// k_fused's forward part: one warp transforms blocks_per_warp<BW>()
+// consecutive blocks (rows, then columns, then a coalesced 16-byte copy-out of
+// the contiguous spectra), which stay in the warp's shared memory.
+template <int BW, int BH, typename T>
+__device__ __forceinline__ void forward_cta(const ForwardArgs& a, int cta) {
   constexpr int NH = BW / 2 + 1, HC = BW / 2, NBW = blocks_per_warp<BW>(), BINS = BH * NH;
   extern __shared__ __align__(16) float2 smem2[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* S = smem2 + warp * NBW * BINS;
   const Geom& g = a.g;
+  const ArgsFwd win{a};
   const int blk0 = (cta * kWarps + warp) * NBW;
   if (blk0 >= g.nblocks) return;
-  constexpr int RPL = (NBW * BH + 31) / 32;  // rows per lane
-  constexpr int NV = PREFETCH ? raw_vectors<BW, T>() : 0;
-  if constexpr (NV > 0) {
-    // every row of the lane fetched before the first transform: one load
-    // latency per warp instead of one per row
-    uint4 raw[RPL][NV];
-    bool have[RPL];
-#pragma unroll
-    for (int i = 0; i < RPL; i++) {
-      const int t = lane + 32 * i, b = t / BH, y = t - b * BH;
-      have[i] = false;
-      if (t < NBW * BH && blk0 + b < g.nblocks) {
-        int x0, row;
-        const T* srow = fwd_row_src<T>(a, win, blk0 + b, y, &x0, &row);
-        const T* p = srow + x0;
-        if (x0 >= 0 && x0 + BW <= g.W && (reinterpret_cast<uintptr_t>(p) & 15) == 0 &&
-            FFT3D_IN(row >= 0 && row < g.H, a.err)) {
-#pragma unroll
-          for (int v = 0; v < NV; v++) raw[i][v] = __ldg(reinterpret_cast<const uint4*>(p) + v);
-          have[i] = true;
-        }
-      }
-    }
-#if FFT3D_FWD_ROW_LOOP
-    // one copy of the row transform in the code: the lane's rows walked by a
-    // loop, each row's prefetched vectors picked by selects (no local memory)
-#pragma unroll 1
-    for (int i = 0; i < RPL; i++) {
-      const int t = lane + 32 * i, b = t / BH, y = t - b * BH;
-      uint4 rr[NV];
-      bool hv = false;
-#pragma unroll
-      for (int q = 0; q < RPL; q++) {
-        if (q == i) hv = have[q];
-#pragma unroll
-        for (int v = 0; v < NV; v++) rr[v] = q == i ? raw[q][v] : (q == 0 ? raw[0][v] : rr[v]);
-      }
-      if (t < NBW * BH && blk0 + b < g.nblocks)
-        fwd_row<BW, BH, T, PREFETCH>(a, win, blk0 + b, y, S + b * BINS, hv ? rr : nullptr);
-    }
-#else
-#pragma unroll
-    for (int i = 0; i < RPL; i++) {
-      const int t = lane + 32 * i, b = t / BH, y = t - b * BH;
-      if (t < NBW * BH && blk0 + b < g.nblocks)
-        fwd_row<BW, BH, T, PREFETCH>(a, win, blk0 + b, y, S + b * BINS, have[i] ? raw[i] : nullptr);
-    }
-#endif
-  } else {
-    for (int t = lane; t < NBW * BH; t += 32) {
-      const int b = t / BH, y = t - b * BH;
-      if (blk0 + b < g.nblocks) fwd_row<BW, BH, T, PREFETCH>(a, win, blk0 + b, y, S + b * BINS, nullptr);
-    }
+  for (int t = lane; t < NBW * BH; t += 32) {
+    const int b = t / BH, y = t - b * BH;
+    if (blk0 + b < g.nblocks) fwd_row<BW, BH, T>(a, win, blk0 + b, y, S + b * BINS);
   }
   __syncwarp();
   for (int t = lane; t < NBW * HC; t += 32) {
@@ -419,57 +317,209 @@ __device__ __forceinline__ void forward_cta_w(const ForwardArgs& a, int cta, con
   for (int i = lane; i < nvalid * BINS / 2; i += 32)
     if (FFT3D_IN((size_t)blk0 * BINS / 2 + i < (size_t)g.nblocks * BINS / 2 && win.spec() != nullptr, a.err))
       dst[i] = src[i];
-  __syncwarp();  // S is reused by the warp's next work item
+  __syncwarp();
 }
 
-template <int BW, int BH, typename T, bool PREFETCH = true>
-__device__ __forceinline__ void forward_cta(const ForwardArgs& a, int cta) {
-  forward_cta_w<BW, BH, T, PREFETCH, ArgsFwd>(a, cta, ArgsFwd{a});
-}
+// Blocks of a forward CTA, and its threads: one per column (DC and Nyquist
+// columns count as one), so that the column transforms are one full round
+// and the row pairs of square blocks too (48 x 48: 4 blocks, 96 threads; a
+// warp per block left a quarter of its lanes idle in both).
+template <int BW>
+__host__ __device__ constexpr int fwd_blocks() { return kWarps * blocks_per_warp<BW>(); }
+template <int BW>
+__host__ __device__ constexpr int fwd_threads() { return fwd_blocks<BW>() * (BW / 2); }
 
-template <int BW, int BH, typename T>
-__global__ void __launch_bounds__(kWarps * 32, 5) k_forward(ForwardArgs a) {
-  forward_cta<BW, BH, T>(a, blockIdx.x);
-}
-
-// The new frames of a frame group in one launch: CTA x transforms CTA
-// x % fs.ctas of frame x / fs.ctas (one launch instead of one per frame, so
-// the grid has no per-frame wave tail).
-template <int BW, int BH, typename T>
-__global__ void __launch_bounds__(kWarps * 32, ctas_for(FFT3D_FWD_CTAS, kWarps * fft_smem_bytes<BW, BH>()))
-    k_forward_frames(ForwardArgs a, FwdFrameSet fs) {
-  const int j = blockIdx.x / fs.ctas, c = blockIdx.x - j * fs.ctas;
-  FrameFwd w{nullptr, 0, nullptr};
+// The BW samples at p as 32-bit words: 16-byte loads where p allows, else
+// 4-byte loads of the words that hold them (never past the word of the last
+// sample) and funnel shifts.
+template <typename T, int BW>
+__device__ __forceinline__ void load_words(const T* p, uint32_t (&w)[BW * sizeof(T) / 4]) {
+  constexpr int WORDS = BW * (int)sizeof(T) / 4;
+  static_assert(BW * sizeof(T) % 4 == 0, "whole words");
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  if (WORDS % 4 == 0 && (at & 15) == 0) {
+    const uint4* q = reinterpret_cast<const uint4*>(p);
 #pragma unroll
-  for (int q = 0; q < kMaxFwdFrames; q++)
-    if (q == j) {
-      w.s = fs.src[q];
-      w.st = fs.stride[q];
-      w.sp = fs.spec[q];
+    for (int v = 0; v < WORDS / 4; v++) {
+      const uint4 u = __ldg(q + v);
+      w[4 * v] = u.x, w[4 * v + 1] = u.y, w[4 * v + 2] = u.z, w[4 * v + 3] = u.w;
     }
-  forward_cta_w<BW, BH, T, true, FrameFwd>(a, c, w);
+    return;
+  }
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(at & ~(uintptr_t)3);
+#pragma unroll
+  for (int v = 0; v < WORDS; v++) w[v] = __ldg(q + v);
+  if constexpr (sizeof(T) < 4) {
+    const int shift = 8 * (int)(at & 3);
+    if (shift) {
+      const uint32_t last = __ldg(q + WORDS);
+#pragma unroll
+      for (int v = 0; v < WORDS; v++) w[v] = __funnelshift_r(w[v], v + 1 < WORDS ? w[v + 1] : last, shift);
+    }
+  }
+}
+
+// Sample x of a row's words as a float of 2^23 + sample (8/16-bit samples: one
+// byte permute into the low mantissa bits of 2^23, exact), or the sample itself.
+template <typename T, int WORDS>
+__device__ __forceinline__ float raw_sample(const uint32_t (&w)[WORDS], int x) {
+  if constexpr (sizeof(T) == 1) return __uint_as_float(__byte_perm(w[x >> 2], 0x4B000000u, 0x7540u | (uint32_t)(x & 3)));
+  else if constexpr (sizeof(T) == 2) return __uint_as_float(__byte_perm(w[x >> 1], 0x4B000000u, (x & 1) ? 0x7432u : 0x7410u));
+  else return __uint_as_float(w[x]);
+}
+
+// Forward transform of fwd_blocks<BW>() consecutive blocks per CTA.
+//  rows: a thread takes rows y and y + bh/2 of a block at once, packed
+//   (rfft_pair): gather with mirrored edges, analysis window, r2c; their
+//   spectra go to shared memory interleaved, 16 bytes per bin {A.re, B.re,
+//   A.im, B.im};
+//  columns: a thread takes a column (bh/2 16-byte reads), transforms it and,
+//   when every thread of the block has read its column, writes it back as
+//   (re, im) rows;
+//  a coalesced 16-byte copy-out of the contiguous spectra.
+// Where a block's threads lie in one warp (square blocks of 8, 16 and 32) the
+// stages are separated by __syncwarp, else by CTA barriers.
+// Bound by issue and the FMA pipe: N us per 1080p frame of 32 x 32 blocks (all
+// planes) against 22.0 with one row at a time per lane.
+template <int BW, int BH, typename T, class Win>
+__device__ __forceinline__ void forward_blocks(const ForwardArgs& a, int cta, const Win& win) {
+  constexpr int NH = BW / 2 + 1, HC = BW / 2, HB = BH / 2, BINS = BH * NH, NT = fwd_threads<BW>();
+  constexpr bool WARP = HB == HC && 32 % HC == 0;  // a block's work stays in one warp
+  constexpr int GT = WARP ? 32 : NT, GB = GT / HC;  // threads and blocks of a group that synchronises
+  constexpr int WORDS = BW * (int)sizeof(T) / 4;
+  extern __shared__ __align__(16) float2 smem2[];
+  const Geom& g = a.g;
+  const int grp = threadIdx.x / GT, t = threadIdx.x - grp * GT;
+  const int blk0 = cta * fwd_blocks<BW>() + grp * GB;
+  const int nvalid = min(GB, g.nblocks - blk0);
+  float2* S = smem2 + grp * GB * BINS;
+  auto sync = [] {
+    if constexpr (WARP) __syncwarp();
+    else __syncthreads();
+  };
+  if (WARP && nvalid <= 0) return;
+  for (int i = t; i < GB * HB; i += GT) {
+    const int b = i / HB, y = i - b * HB;
+    if (b >= nvalid) continue;
+    float4* quads = reinterpret_cast<float4*>(S + b * BINS) + y * NH;
+    int x0, rowA, rowB;
+    const T* srcA = fwd_row_src<T>(a, win, blk0 + b, y, &x0, &rowA);
+    const T* srcB = fwd_row_src<T>(a, win, blk0 + b, y + HB, &x0, &rowB);
+    const bool okA = FFT3D_IN(rowA >= 0 && rowA < g.H, a.err), okB = FFT3D_IN(rowB >= 0 && rowB < g.H, a.err);
+    f2x v[BW];
+    const float off = (sizeof(T) < 4 ? 8388608.0f : 0.f) + a.base;  // exact: base <= 2^15
+    const f2x noff = dup2(-off);
+    if (x0 >= 0 && x0 + BW <= g.W && okA && okB) {
+      uint32_t wA[WORDS], wB[WORDS];
+      load_words<T, BW>(srcA + x0, wA);
+      load_words<T, BW>(srcB + x0, wB);
+#pragma unroll
+      for (int x = 0; x < BW; x++) v[x] = pk2(raw_sample<T>(wA, x), raw_sample<T>(wB, x));
+    } else {
+      // mirrored columns: sample by sample through the thread's own part of
+      // the tile (as samples plus the offset that the common path takes off)
+      f2x* own = reinterpret_cast<f2x*>(quads);
+      const float up = sizeof(T) < 4 ? 8388608.0f : 0.f;
+#pragma unroll 8
+      for (int x = 0; x < BW; x++) {
+        const int xi = reflect101(x0 + x, g.W);
+        const bool in = FFT3D_IN(xi >= 0 && xi < g.W, a.err);
+        own[x] = pk2(in && okA ? load_sample<T>(srcA + xi) + up : off, in && okB ? load_sample<T>(srcB + xi) + up : off);
+      }
+#pragma unroll
+      for (int x = 0; x < BW; x++) v[x] = own[x];
+    }
+    const f2x wy = pk2(__ldg(a.wan_y + y), __ldg(a.wan_y + y + HB));
+#pragma unroll
+    for (int x = 0; x < BW; x++)
+      v[x] = mul2_kept(mul2(add2(v[x], noff), *reinterpret_cast<const f2x*>(&a.wx_half[x])), wy);
+    f2x re[NH], im[NH];
+    rfft_pair<BW>(v, re, im);
+#pragma unroll
+    for (int k = 0; k < NH; k++) {
+      const float2 r = up2(re[k]), q = up2(im[k]);
+      quads[k] = make_float4(r.x, r.y, q.x, q.y);
+    }
+  }
+  sync();
+  float2 col[BH];
+  const int cb = t / HC, c = t - cb * HC;
+  const bool mine = cb < nvalid;
+  float2* Sb = S + cb * BINS;
+  if (mine) {
+    const float4* quads = reinterpret_cast<const float4*>(Sb);
+#pragma unroll
+    for (int y = 0; y < HB; y++) {
+      const float4 q = quads[y * NH + c];
+      col[y] = make_float2(q.x, q.z);
+      col[y + HB] = make_float2(q.y, q.w);
+      if (c == 0) {  // real columns 0 and bw/2 as one complex sequence
+        const float4 n = quads[y * NH + HC];
+        col[y].y = n.x;
+        col[y + HB].y = n.y;
+      }
+    }
+  }
+  sync();
+  if (mine) {
+    cfft<BH, -1>(col);
+    if (c == 0) {
+#pragma unroll
+      for (int h = 0; h < BH; h++) {
+        const float2 zh = col[h], zm = cconj(col[(BH - h) % BH]);
+        Sb[h * NH] = make_float2(0.5f * (zh.x + zm.x), 0.5f * (zh.y + zm.y));
+        const float2 d = csub(zh, zm);
+        Sb[h * NH + HC] = make_float2(0.5f * d.y, -0.5f * d.x);
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < BH; h++) Sb[h * NH + c] = col[h];
+    }
+  }
+  sync();
+  float4* dst = reinterpret_cast<float4*>(win.spec() + (size_t)blk0 * BINS);
+  const float4* src = reinterpret_cast<const float4*>(S);
+  for (int i = t; i < nvalid * BINS / 2; i += GT)
+    if (FFT3D_IN((size_t)blk0 * BINS / 2 + i < (size_t)g.nblocks * BINS / 2 && win.spec() != nullptr, a.err))
+      dst[i] = src[i];
+}
+
+// Registers of the forward kernels: two packed rows of 32 samples are 64
+// registers, of 48 samples 96.
+template <int BW, int BH>
+__host__ __device__ constexpr int fwd_ctas(int extra) {
+  return ctas_for((BW > 32 || BH > 32 ? 15 : 20) * 32 / fwd_threads<BW>(), fwd_blocks<BW>() * BH * (BW / 2 + 1) * 8 + extra);
+}
+template <int BW, int BH>
+__host__ __device__ constexpr int fwd_smem() { return fwd_blocks<BW>() * BH * (BW / 2 + 1) * 8; }
+
+// The new frames of one or more output frames in one launch: CTA x transforms
+// CTA x % fs.ctas of frame x / fs.ctas (one launch instead of one per frame,
+// so the grid has no per-frame wave tail).
+template <int BW, int BH, typename T>
+__global__ void __launch_bounds__(fwd_threads<BW>(), (fwd_ctas<BW, BH>(0)))
+    k_forward_frames(const __grid_constant__ ForwardArgs a, const __grid_constant__ FwdFrameSet fs) {
+  const int j = blockIdx.x / fs.ctas, c = blockIdx.x - j * fs.ctas;
+  forward_blocks<BW, BH, T>(a, c, FrameFwd{fs.src[j], fs.stride[j], fs.spec[j]});
 }
 
 // Batched forward: work item i = (plane, CTA of that plane); the grid walks
 // the items (persistent when the grid is smaller than the item count).
 template <int BW, int BH, typename T>
-__global__ void __launch_bounds__(kWarps * 32,
-                                  ctas_for(FFT3D_FWD_CTAS, kWarps * fft_smem_bytes<BW, BH>() + (int)sizeof(ForwardArgs)))
-    k_forward_batch(const ForwardArgs* __restrict__ args,
-                                                                 const int2* __restrict__ items, int nitems) {
+__global__ void __launch_bounds__(fwd_threads<BW>(), (fwd_ctas<BW, BH>((int)sizeof(ForwardArgs))))
+    k_forward_batch(const ForwardArgs* __restrict__ args, const int2* __restrict__ items, int nitems) {
   // the item's arguments staged in shared memory: the body's stores cannot
-  // alias them, they cost no registers, and the body can take the per-plane
-  // kernel's row prefetch (x window read from the staged arguments)
+  // alias them, and they cost no registers
   __shared__ __align__(16) ForwardArgs sa;
   static_assert(sizeof(ForwardArgs) % 4 == 0, "word copy");
   for (int i = blockIdx.x; i < nitems; i += gridDim.x) {
     const int2 it = items[i];
-    __syncthreads();  // every warp is done with the previous item's arguments
+    __syncthreads();  // every warp is done with the previous item's arguments and tiles
     const int* src = reinterpret_cast<const int*>(args + it.x);
     int* dst = reinterpret_cast<int*>(&sa);
     for (int w = threadIdx.x; w < (int)(sizeof(ForwardArgs) / 4); w += blockDim.x) dst[w] = src[w];
     __syncthreads();
-    forward_cta<BW, BH, T, true>(sa, it.y);
+    forward_blocks<BW, BH, T>(sa, it.y, ArgsFwd{sa});
   }
 }
 
@@ -697,43 +747,6 @@ __device__ __forceinline__ float2 sharpen_bin(const InverseArgs& a, float2 v, co
 
 // ---------------------------------------------------------------- filters, two bins at a time
 
-// Two floats in one 64-bit register pair, for the packed f32x2 instructions
-// (each lane rounds like the scalar operation). Held as one 64-bit value and
-// worked on with PTX: the same arithmetic on float2 and its intrinsics cost 50
-// register moves per bin pair and frame at bt = 5 (188 instructions instead of
-// 128), because the halves are then allocated one by one.
-using f2x = unsigned long long;
-__device__ __forceinline__ f2x pk2(float lo, float hi) {
-  f2x r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ f2x dup2(float v) { return pk2(v, v); }
-__device__ __forceinline__ float2 up2(f2x v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ f2x add2(f2x a, f2x b) {
-  f2x r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2x sub2(f2x a, f2x b) {
-  f2x r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2x mul2(f2x a, f2x b) {
-  f2x r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2x fma2(f2x a, f2x b, f2x c) {
-  f2x r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 __device__ __forceinline__ f2x rcp2(f2x v) {
   const float2 u = up2(v);
   return pk2(rcp_nrm(u.x), rcp_nrm(u.y));
@@ -778,14 +791,6 @@ __device__ __forceinline__ float4 bins_of(const Pair& p) {
   return make_float4(re.x, im.x, re.y, im.y);
 }
 __device__ __forceinline__ Pair padd(const Pair& x, const Pair& y) { return Pair{add2(x.re, y.re), add2(x.im, y.im)}; }
-// x * s with products that stay products: ptxas contracts a packed multiply
-// into a packed add that follows (explicit rounding or not), which would round
-// once where filter_vals and sharpen_bin round twice; two scalar multiplies
-// are left alone, at the same cost on the FMA pipe.
-__device__ __forceinline__ f2x mul2_kept(f2x v, f2x s) {
-  const float2 a = up2(v), b = up2(s);
-  return pk2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
-}
 __device__ __forceinline__ Pair pscale_kept(const Pair& x, f2x s) { return Pair{mul2_kept(x.re, s), mul2_kept(x.im, s)}; }
 __device__ __forceinline__ Pair psub(const Pair& x, const Pair& y) { return Pair{sub2(x.re, y.re), sub2(x.im, y.im)}; }
 __device__ __forceinline__ Pair pscale(const Pair& x, f2x s) { return Pair{mul2(x.re, s), mul2(x.im, s)}; }
@@ -1997,7 +2002,7 @@ __global__ void __launch_bounds__(kBulkWarps * 32) k_filter_inverse_bulk(Inverse
 template <int BW, int BH, typename T, int MODE>
 __global__ void __launch_bounds__(kWarps * 32, 6) k_fused(FusedArgs A) {
   const int n = fft_ctas<BW, BH>(A.v.g.nblocks);
-  forward_cta<BW, BH, T, false>(A.f, A.v.reverse ? n - 1 - (int)blockIdx.x : (int)blockIdx.x);
+  forward_cta<BW, BH, T>(A.f, A.v.reverse ? n - 1 - (int)blockIdx.x : (int)blockIdx.x);
   filter_inverse_cta<BW, BH, MODE, true>(A.v, blockIdx.x);
 }
 
@@ -2009,22 +2014,19 @@ int fft_grid(int nblocks) {
 }
 
 // Batched launches of one kernel variant over many planes (see k_forward_batch).
+template <int BW, int BH, typename T>
+cudaError_t fwd_batch_typed(const BatchLaunch& l, cudaStream_t s) {
+  const cudaError_t e = fft3d::smem_attr(k_forward_batch<BW, BH, T>, fwd_smem<BW, BH>());
+  if (e != cudaSuccess) return e;
+  k_forward_batch<BW, BH, T><<<l.grid, fwd_threads<BW>(), fwd_smem<BW, BH>(), s>>>(static_cast<const ForwardArgs*>(l.args),
+                                                                                   l.items, l.nitems);
+  return cudaGetLastError();
+}
 template <int BW, int BH>
 cudaError_t fwd_batch(const BatchLaunch& l, int bytes, cudaStream_t s) {
-  const int smem = kWarps * fft_smem_bytes<BW, BH>();
-  const auto* args = static_cast<const ForwardArgs*>(l.args);
-  cudaError_t e = cudaSuccess;
-  if (bytes == 1) {
-    e = fft3d::smem_attr(k_forward_batch<BW, BH, uint8_t>, smem);
-    if (e == cudaSuccess) k_forward_batch<BW, BH, uint8_t><<<l.grid, kWarps * 32, smem, s>>>(args, l.items, l.nitems);
-  } else if (bytes == 2) {
-    e = fft3d::smem_attr(k_forward_batch<BW, BH, uint16_t>, smem);
-    if (e == cudaSuccess) k_forward_batch<BW, BH, uint16_t><<<l.grid, kWarps * 32, smem, s>>>(args, l.items, l.nitems);
-  } else {
-    e = fft3d::smem_attr(k_forward_batch<BW, BH, float>, smem);
-    if (e == cudaSuccess) k_forward_batch<BW, BH, float><<<l.grid, kWarps * 32, smem, s>>>(args, l.items, l.nitems);
-  }
-  return e != cudaSuccess ? e : cudaGetLastError();
+  if (bytes == 1) return fwd_batch_typed<BW, BH, uint8_t>(l, s);
+  if (bytes == 2) return fwd_batch_typed<BW, BH, uint16_t>(l, s);
+  return fwd_batch_typed<BW, BH, float>(l, s);
 }
 
 template <int BW, int BH, int MODE>
@@ -2063,7 +2065,7 @@ int occupancy_of(int which, int mode_or_bytes) {
   const int smem = kWarps * fft_smem_bytes<BW, BH>();
   int n = 0;
   if (which == 0) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_forward_batch<BW, BH, uint8_t>, kWarps * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_forward_batch<BW, BH, uint8_t>, fwd_threads<BW>(), fwd_smem<BW, BH>());
   } else if (which == 3) {
     const int gsmem = group_smem_bytes<BW, BH>(run_tiles<BW, BH, 5, run_staged<BW, BH, 5>()>()) + (int)sizeof(GroupRun);
     fft3d::smem_attr(k_filter_inverse_group_batch<BW, BH, 5>, gsmem);
@@ -2083,22 +2085,31 @@ int occupancy_of(int which, int mode_or_bytes) {
   return n > 0 ? n : 1;
 }
 
+template <int BW, int BH, typename T>
+cudaError_t fwd_typed(const ForwardArgs& a, const FwdFrameSet& fs, cudaStream_t s) {
+  const cudaError_t e = fft3d::smem_attr(k_forward_frames<BW, BH, T>, fwd_smem<BW, BH>());
+  if (e != cudaSuccess) return e;
+  k_forward_frames<BW, BH, T><<<fs.ctas * fs.count, fwd_threads<BW>(), fwd_smem<BW, BH>(), s>>>(a, fs);
+  return cudaGetLastError();
+}
+template <int BW, int BH>
+cudaError_t fwd_frames(const ForwardArgs& a, const FwdFrameSet& fs, int bytes, cudaStream_t s) {
+  if (fs.count < 1 || fs.count > kMaxFwdFrames) return cudaErrorInvalidValue;
+  FwdFrameSet f = fs;
+  f.ctas = (a.g.nblocks + fwd_blocks<BW>() - 1) / fwd_blocks<BW>();
+  if (bytes == 1) return fwd_typed<BW, BH, uint8_t>(a, f, s);
+  if (bytes == 2) return fwd_typed<BW, BH, uint16_t>(a, f, s);
+  return fwd_typed<BW, BH, float>(a, f, s);
+}
+// one frame: a set of one
 template <int BW, int BH>
 cudaError_t fwd_sized(const ForwardArgs& a, int bytes, cudaStream_t s) {
-  const int smem = kWarps * fft_smem_bytes<BW, BH>();
-  const int grid = fft_grid<BW, BH>(a.g.nblocks);
-  cudaError_t e = cudaSuccess;
-  if (bytes == 1) {
-    e = fft3d::smem_attr(k_forward<BW, BH, uint8_t>, smem);
-    if (e == cudaSuccess) k_forward<BW, BH, uint8_t><<<grid, kWarps * 32, smem, s>>>(a);
-  } else if (bytes == 2) {
-    e = fft3d::smem_attr(k_forward<BW, BH, uint16_t>, smem);
-    if (e == cudaSuccess) k_forward<BW, BH, uint16_t><<<grid, kWarps * 32, smem, s>>>(a);
-  } else {
-    e = fft3d::smem_attr(k_forward<BW, BH, float>, smem);
-    if (e == cudaSuccess) k_forward<BW, BH, float><<<grid, kWarps * 32, smem, s>>>(a);
-  }
-  return e != cudaSuccess ? e : cudaGetLastError();
+  FwdFrameSet fs{};
+  fs.src[0] = a.src;
+  fs.stride[0] = a.src_stride;
+  fs.spec[0] = a.spec;
+  fs.count = 1;
+  return fwd_frames<BW, BH>(a, fs, bytes, s);
 }
 
 // Blocks per CTA of a run whose block takes `count` tiles, over nblocks
@@ -2208,27 +2219,6 @@ cudaError_t fused_sized(const FusedArgs& a, int mode, int bytes, cudaStream_t s)
   if (bytes == 1) return fused_typed<BW, BH, uint8_t>(a, mode, s);
   if (bytes == 2) return fused_typed<BW, BH, uint16_t>(a, mode, s);
   return cudaErrorNotSupported;  // float samples use the unfused path
-}
-
-template <int BW, int BH>
-cudaError_t fwd_frames(const ForwardArgs& a, const FwdFrameSet& fs, int bytes, cudaStream_t s) {
-  if (fs.count < 1 || fs.count > kMaxFwdFrames) return cudaErrorInvalidValue;
-  const int smem = kWarps * fft_smem_bytes<BW, BH>();
-  FwdFrameSet f = fs;
-  f.ctas = fft_grid<BW, BH>(a.g.nblocks);
-  const int grid = f.ctas * f.count;
-  cudaError_t e = cudaSuccess;
-  if (bytes == 1) {
-    e = fft3d::smem_attr(k_forward_frames<BW, BH, uint8_t>, smem);
-    if (e == cudaSuccess) k_forward_frames<BW, BH, uint8_t><<<grid, kWarps * 32, smem, s>>>(a, f);
-  } else if (bytes == 2) {
-    e = fft3d::smem_attr(k_forward_frames<BW, BH, uint16_t>, smem);
-    if (e == cudaSuccess) k_forward_frames<BW, BH, uint16_t><<<grid, kWarps * 32, smem, s>>>(a, f);
-  } else {
-    e = fft3d::smem_attr(k_forward_frames<BW, BH, float>, smem);
-    if (e == cudaSuccess) k_forward_frames<BW, BH, float><<<grid, kWarps * 32, smem, s>>>(a, f);
-  }
-  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <int BW, int BH, int MODE>
