@@ -69,6 +69,8 @@ __device__ __forceinline__ float rsqrt_nrm(float x) {
   return y;
 }
 
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
 // n / d for 0 <= n < 2^24, d > 0 and a quotient below 2^20 (pixel and block
 // coordinates over a block step or a row length), exact: the estimate
 // n * (1/d) is within (n / d) * 2^-21 < 0.5 of n / d (reciprocal <= 2 ulp,
@@ -376,11 +378,12 @@ __device__ __forceinline__ float raw_sample(const uint32_t (&w)[WORDS], int x) {
 //  columns: a thread takes a column (bh/2 16-byte reads), transforms it and,
 //   when every thread of the block has read its column, writes it back as
 //   (re, im) rows;
-//  a coalesced 16-byte copy-out of the contiguous spectra.
+//  one bulk copy of the contiguous spectra to global memory per group.
 // Where a block's threads lie in one warp (square blocks of 8, 16 and 32) the
 // stages are separated by __syncwarp, else by CTA barriers.
-// Bound by issue and the FMA pipe: N us per 1080p frame of 32 x 32 blocks (all
-// planes) against 22.0 with one row at a time per lane.
+// Bound by issue and shared-memory traffic: 18.7 us per 1080p frame of 32 x 32
+// blocks (all planes; 818 instructions per block with the copy-out by 16-byte
+// loads and stores, then 21.1 us) against 21.2 (1166) with one row at a time.
 template <int BW, int BH, typename T, class Win>
 __device__ __forceinline__ void forward_blocks(const ForwardArgs& a, int cta, const Win& win) {
   constexpr int NH = BW / 2 + 1, HC = BW / 2, HB = BH / 2, BINS = BH * NH, NT = fwd_threads<BW>();
@@ -476,12 +479,15 @@ __device__ __forceinline__ void forward_blocks(const ForwardArgs& a, int cta, co
       for (int h = 0; h < BH; h++) Sb[h * NH + c] = col[h];
     }
   }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   sync();
-  float4* dst = reinterpret_cast<float4*>(win.spec() + (size_t)blk0 * BINS);
-  const float4* src = reinterpret_cast<const float4*>(S);
-  for (int i = t; i < nvalid * BINS / 2; i += GT)
-    if (FFT3D_IN((size_t)blk0 * BINS / 2 + i < (size_t)g.nblocks * BINS / 2 && win.spec() != nullptr, a.err))
-      dst[i] = src[i];
+  if (t == 0 && nvalid > 0 && FFT3D_IN(blk0 + nvalid <= g.nblocks && win.spec() != nullptr, a.err)) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(win.spec() + (size_t)blk0 * BINS),
+                 "r"(smem_addr(S)), "r"(nvalid * BINS * 8)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the tiles are read before the CTA leaves them
+  }
 }
 
 // Registers of the forward kernels: two packed rows of 32 samples are 64
@@ -809,7 +815,9 @@ __device__ __forceinline__ Pair psum2(const Pair& x, f2x fx, const Pair& y, f2x 
 
 // filter_vals of a Wiener 3D mode for a pair; w: the pair in the window's
 // frames, grid: the pair's gridsample (zeros without degrid), gf: the block's
-// grid fraction, nn: minus the pair's noise powers.
+// grid fraction, nn: minus the pair's noise powers. (The last scaling is kept
+// apart from the subtraction that a sharpen pass begins with; a half and a
+// quarter are exact either way.)
 template <int MODE>
 __device__ __forceinline__ Pair filter_pair(const Pair (&w)[5], const Pair& grid, float gf, f2x nn, float ll) {
   static_assert(MODE >= 2 && MODE <= 5, "Wiener 3D");
@@ -823,7 +831,7 @@ __device__ __forceinline__ Pair filter_pair(const Pair (&w)[5], const Pair& grid
     const Pair fc = psub(padd(cur, pn), g);
     const Pair h = pfma(pn, kc(kMinusHalf), cur), d = pscale_kept(psub(w[1], w[3]), kc(kSin120));
     const Pair fp = psub_i(h, d), fn = padd_i(h, d);
-    return pscale(padd(pfma(fn, factor(fn), psum2(fc, factor(fc), fp, factor(fp))), g), kc(kThird));
+    return pscale_kept(padd(pfma(fn, factor(fn), psum2(fc, factor(fc), fp, factor(fp))), g), kc(kThird));
   } else if constexpr (MODE == 4) {
     const Pair cp = padd(cur, w[0]), cm = psub(cur, w[0]), pn = padd(w[1], w[3]), d = psub(w[1], w[3]);
     const Pair fp2 = psub(cp, pn), fc = psub(padd(cp, pn), g);
@@ -841,7 +849,7 @@ __device__ __forceinline__ Pair filter_pair(const Pair (&w)[5], const Pair& grid
     const Pair fp = psub_i(s2, t2), fn = padd_i(s2, t2);
     const Pair fc = psub(padd(padd(a2, a1), cur), g);
     const Pair sum = padd(psum2(fp2, factor(fp2), fp, factor(fp)), psum2(fc, factor(fc), fn, factor(fn)));
-    return pscale(padd(pfma(fn2, factor(fn2), sum), g), kc(kFifth));
+    return pscale_kept(padd(pfma(fn2, factor(fn2), sum), g), kc(kFifth));
   }
 }
 
@@ -1433,7 +1441,6 @@ __device__ __forceinline__ void overlap_add_px4(const OlaArgs& a, int x0, int k)
 
 constexpr int kBulkSpin = 1 << 22;  // bounded mbarrier wait (then error flag 2)
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool bulk_wait(uint64_t* bar, uint32_t parity) {
   uint32_t done = 0;
   for (int it = 0; it < kBulkSpin && !done; it++)
@@ -1487,13 +1494,15 @@ __device__ __forceinline__ float4 group_load(const InverseArgs& a, const Tempora
 
 // Bins bin, bin + 1 of the block at `off` through all the run's frames, in
 // order: Wiener 3D with the window of MODE frames in registers (each spectrum
-// read once, the next frame's bins loaded one frame ahead), or Kalman with
-// the state in registers. load(s): the pair in the run's window spectrum s;
-// gfs: the grid fraction of the block's first frame, tile: the pair's place in
-// its tile; both `stride` tiles apart from frame to frame.
+// read once, the next frame's bins loaded one frame ahead) and the separate
+// sharpen/dehalo pass, or Kalman with the state in registers. load(s): the
+// pair in the run's window spectrum s; gfs, gsh: the grid fractions of the
+// block's first frame, before and after the filter, tile: the pair's place in
+// its tile; all `stride` tiles apart from frame to frame.
 template <int MODE, int BINS, class Load>
 __device__ __forceinline__ void group_filter_pair(const InverseArgs& a, size_t off, int bin, int count,
-                                                  const float* gfs, float2* tile, int stride, const Load& load) {
+                                                  const float* gfs, const float* gsh, float2* tile, int stride,
+                                                  const Load& load) {
   if constexpr (MODE == MODE_KALMAN) {
     float4 lv;
     float2 cv, cp;
@@ -1525,6 +1534,9 @@ __device__ __forceinline__ void group_filter_pair(const InverseArgs& a, size_t o
     constexpr int LO = win_lo<MODE>(), HI = win_hi<MODE>(), NW = HI - LO + 1;
     const Pair grid = pair_grid(a, bin);
     const f2x nn = pair_noise<MODE>(a, off, bin);
+    const bool sh = a.c.do_sharpen;
+    const f2x wsh = pair_weights(a.t.wsharpen, sh && a.c.use_sharpen, bin),
+              wdh = pair_weights(a.t.wdehalo, sh && a.c.use_dehalo, bin);
     // spectrum s (frame n0 - 2 + s) lives in r[s % NW]; frame j reads
     // s = j + LO .. j + HI; with j = j0 + u and j0 a multiple of NW every
     // index below is a compile-time constant
@@ -1542,7 +1554,8 @@ __device__ __forceinline__ void group_filter_pair(const InverseArgs& a, size_t o
         Pair w[5];
 #pragma unroll
         for (int k = 0; k < 5; k++) w[k] = r[(u + (k >= LO && k <= HI ? k : LO)) % NW];
-        const Pair v = filter_pair<MODE>(w, grid, gfs[j * stride], nn, a.c.lowlimit);
+        Pair v = filter_pair<MODE>(w, grid, gfs[j * stride], nn, a.c.lowlimit);
+        if (a.c.do_sharpen) v = sharpen_pair(a, v, grid, wsh, wdh, gsh[j * stride]);
         *reinterpret_cast<float4*>(tile + j * stride * BINS) = bins_of(v);
         if (++j == count) return;
       }
@@ -1634,18 +1647,16 @@ __host__ __device__ constexpr int run_ctas(int extra) {
 //     the filter then works in place, since frame j's window begins with the
 //     spectrum whose tile it overwrites and one thread takes a pair through
 //     all frames. Otherwise the filter reads the spectra from global memory;
-//  1. the grid fraction of each tile (its block's DC in its frame), then the
-//     filter. Wiener 3D runs of 2 frames and more, and Kalman: each thread
-//     takes two neighbouring bins and walks the run's frames in order, its
-//     window in registers, so that each of the block's count + MODE - 1
-//     window spectra is read once for the run (and a Kalman state once);
-//     pairs beyond the last whole round of the CTA's threads, and all pairs
-//     of shorter or window-less runs, are spread over all threads as single
-//     (pair, frame) items. The thread that holds a tile's DC publishes the
-//     filtered DC;
-//  2. the separate sharpen/dehalo pass (src/code_impl/Sharpen.cpp:13-63), its
-//     grid fraction from each tile's filtered DC, the pair's tables loaded
-//     once for all frames;
+//  1. the grid fractions of each tile (its block's DC in its frame, and that
+//     DC filtered, for the sharpen pass), then the filter with the separate
+//     sharpen/dehalo pass. Wiener 3D runs of 2 frames and more, and Kalman:
+//     each thread takes two neighbouring bins and walks the run's frames in
+//     order, its window in registers, so that each of the block's count +
+//     MODE - 1 window spectra is read once for the run (and a Kalman state
+//     once); pairs beyond the last whole round of the CTA's threads, and all
+//     pairs of shorter or window-less runs, are spread over all threads as
+//     single (pair, frame) items;
+//  2. Kalman only: the sharpen/dehalo pass, once the filtered DCs are known;
 //  3. the inverse column DFTs of every tile (DC and Nyquist columns as one
 //     complex transform), 4. the c2r rows, 5. coalesced stores of the
 //     time-domain blocks.
@@ -1692,52 +1703,65 @@ __device__ __forceinline__ bool filter_inverse_group_cta(const InverseArgs& a, c
     if constexpr (STAGED) return *reinterpret_cast<const float4*>(S + ((s - LO) * nbv + b) * BINS + bin);
     else return group_load(a, ts, s, off0 + b * BINS, bin);
   };
-  // 1. grid fraction of each tile, and the pairs left after the whole rounds
-  //    of a walk (read here, before any tile is overwritten)
-  if (MODE >= 1 && t < tiles && landed) {
-    const int j = div_small(t, nbv), b = t - j * nbv;
-    float dc = 0.f;
-    if constexpr (STAGED) dc = S[((j + 2 - LO) * nbv + b) * BINS].x;
-    else if (FFT3D_IN(ts.spec[j + 2] != nullptr && blk0 + b < a.g.nblocks, a.err)) dc = __ldg(&ts.spec[j + 2][off0 + b * BINS].x);
-    gfs[t] = a.c.degrid * dc / gs0;
-  }
   constexpr bool WALK = MODE == MODE_KALMAN || MODE >= 2;
   const bool walk = MODE == MODE_KALMAN || (MODE >= 2 && count > 1);
   int full = walk ? npairs : 0;
   if (MODE >= 2 && walk && (npairs % NT) * count <= NT) full = npairs / NT * NT;
+  auto finish = [&](float4 v, int bin, float gf) {  // the separate sharpen/dehalo pass, src/code_impl/Sharpen.cpp:13-63
+    if (MODE != MODE_KALMAN && a.c.do_sharpen)
+      v = bins_of(sharpen_pair(a, pair_of(v), pair_grid(a, bin), pair_weights(a.t.wsharpen, a.c.use_sharpen, bin),
+                               pair_weights(a.t.wdehalo, a.c.use_dehalo, bin), gf));
+    return v;
+  };
+  // 1. pass 0: a thread per tile, bins 0 and 1: the tile's grid fraction (its
+  //    DC) and, for the sharpen pass, the filtered DC's. Pass 1: a thread per
+  //    pair and frame of the pairs left after the whole rounds of a walk,
+  //    read before the barrier (no tile is overwritten yet), filtered after
   float4 r[5];
-  int rj = 0, rp = 0;  // this thread's item of the rest: frame, pair
-  bool item = false;
-  if constexpr (MODE >= 2) {
-    const int rest = npairs - full;
-    if (walk && t < rest * count) {
-      rj = div_small(t, rest);
-      rp = full + t - rj * rest;
-      item = true;
-      const int b = rp / PAIRS, bin = 2 * (rp - b * PAIRS);
+  if constexpr (MODE != MODE_KALMAN) {
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {
+      const int rest = pass == 0 ? nbv : (walk ? npairs - full : 0);
+      const bool item = t < rest * count;
+      int j = 0, p = 0;
+      if (item) {
+        j = div_small(t, rest);
+        p = t - j * rest;
+        p = pass == 0 ? p * PAIRS : full + p;
+      }
+      const int b = p / PAIRS, bin = 2 * (p - b * PAIRS), tile = j * nbv + b;
+      if (item && landed) {
 #pragma unroll
-      for (int k = LO; k <= HI; k++) r[k] = load(rj + k, b, bin);
+        for (int k = LO; k <= HI; k++) r[k] = load(j + k, b, bin);
+      }
+      if (pass == 1) {
+        if constexpr (STAGED) {
+          if (__syncthreads_or(landed ? 0 : 1)) {
+            // the copies never completed: flag it, give them one more bounded
+            // wait (they target this CTA's shared memory), and stop
+            if (t == 0 && a.err) atomicOr(a.err, 2);
+            bulk_wait(bar, phase);
+            return false;
+          }
+        } else {
+          __syncthreads();
+        }
+      }
+      if (item && landed) {
+        const float gf = pass == 0 ? a.c.degrid * r[2].x / gs0 : gfs[tile];
+        if (pass == 1 || a.c.do_sharpen) {
+          const float4 v = group_filter_one<MODE>(a, off0 + b * BINS, bin, r, gf);
+          if (pass == 0) gsh[tile] = a.c.degrid * v.x / gs0;
+          else *reinterpret_cast<float4*>(S + tile * BINS + bin) = finish(v, bin, gsh[tile]);
+        }
+        if (pass == 0) gfs[tile] = gf;
+      }
     }
-  }
-  if constexpr (STAGED) {
+  } else if constexpr (STAGED) {
     if (__syncthreads_or(landed ? 0 : 1)) {
-      // the copies never completed: flag it, give them one more bounded wait
-      // (they target this CTA's shared memory), and stop
       if (t == 0 && a.err) atomicOr(a.err, 2);
       bulk_wait(bar, phase);
       return false;
-    }
-  } else {
-    __syncthreads();
-  }
-  auto put = [&](int tile, int bin, const float4& v) {
-    *reinterpret_cast<float4*>(S + tile * BINS + bin) = v;
-    if (a.c.do_sharpen && bin == 0) gsh[tile] = a.c.degrid * v.x / gs0;  // the sharpen pass's grid fraction
-  };
-  if constexpr (MODE >= 2) {
-    if (item) {
-      const int b = rp / PAIRS, bin = 2 * (rp - b * PAIRS), tile = rj * nbv + b;
-      put(tile, bin, group_filter_one<MODE>(a, off0 + b * BINS, bin, r, gfs[tile]));
     }
   }
   using Cursor = PairCursor<BINS, NT>;
@@ -1745,9 +1769,9 @@ __device__ __forceinline__ bool filter_inverse_group_cta(const InverseArgs& a, c
     Cursor c(t);
     for (int q = t; q < full; q += NT, c.step()) {
       const int b = c.b, bin = c.bin;
-      group_filter_pair<MODE, BINS>(a, off0 + b * BINS, bin, count, gfs + b, S + 2 * q, nbv,
+      group_filter_pair<MODE, BINS>(a, off0 + b * BINS, bin, count, gfs + b, gsh + b, S + 2 * q, nbv,
                                     [&](int s) { return load(s, b, bin); });
-      if (a.c.do_sharpen && bin == 0)
+      if (MODE == MODE_KALMAN && a.c.do_sharpen && bin == 0)
         for (int j = 0; j < count; j++) gsh[j * nbv + b] = a.c.degrid * S[(j * nbv + b) * BINS].x / gs0;
     }
   }
@@ -1771,31 +1795,23 @@ __device__ __forceinline__ bool filter_inverse_group_cta(const InverseArgs& a, c
         c.step();
         while (c.b >= (cj + 1) * nbv) cj++;
         if (q + NT < total) fetch();
-        put(tile, bin, group_filter_one<MODE>(a, off0 + b * BINS, bin, r, MODE >= 1 ? gfs[tile] : 0.f));
+        const float4 v = group_filter_one<MODE>(a, off0 + b * BINS, bin, r, MODE >= 1 ? gfs[tile] : 0.f);
+        *reinterpret_cast<float4*>(S + tile * BINS + bin) = finish(v, bin, a.c.do_sharpen ? gsh[tile] : 0.f);
       }
     }
   }
   __syncthreads();
-  // 2. sharpen/dehalo: whole rounds of bin pairs with the pair's tables
-  //    loaded once for all frames, then the remaining pairs as (pair, frame)
-  //    items
-  if (a.c.do_sharpen) {
-    auto one = [&](float2* at, const Pair& grid, f2x wsh, f2x wdh, float gf) {
-      float4* q = reinterpret_cast<float4*>(at);
-      *q = bins_of(sharpen_pair(a, pair_of(*q), grid, wsh, wdh, gf));
-    };
-    const int whole = npairs * count <= NT ? 0 : npairs / NT * NT, rest = npairs - whole;
+  // 2. Kalman's sharpen/dehalo pass (its filtered DCs are known only now)
+  if (MODE == MODE_KALMAN && a.c.do_sharpen) {
     Cursor c(t);
-    for (int q = t; q < whole; q += NT, c.step()) {
+    for (int q = t; q < npairs; q += NT, c.step()) {
       const Pair grid = pair_grid(a, c.bin);
       const f2x wsh = pair_weights(a.t.wsharpen, a.c.use_sharpen, c.bin),
                 wdh = pair_weights(a.t.wdehalo, a.c.use_dehalo, c.bin);
-      for (int j = 0; j < count; j++) one(S + j * nbv * BINS + 2 * q, grid, wsh, wdh, gsh[j * nbv + c.b]);
-    }
-    for (int i = t; i < rest * count; i += NT) {
-      const int j = div_small(i, rest), p = whole + i - j * rest, b = p / PAIRS, bin = 2 * (p - b * PAIRS);
-      one(S + j * nbv * BINS + 2 * p, pair_grid(a, bin), pair_weights(a.t.wsharpen, a.c.use_sharpen, bin),
-          pair_weights(a.t.wdehalo, a.c.use_dehalo, bin), gsh[j * nbv + b]);
+      for (int j = 0; j < count; j++) {
+        float4* at = reinterpret_cast<float4*>(S + j * nbv * BINS + 2 * q);
+        *at = bins_of(sharpen_pair(a, pair_of(*at), grid, wsh, wdh, gsh[j * nbv + c.b]));
+      }
     }
     __syncthreads();
   }
