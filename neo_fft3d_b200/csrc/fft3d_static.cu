@@ -29,6 +29,7 @@
 //  * the address and the twiddle tables are kept per device number for the
 //    life of the process: do not use the call across a cudaDeviceReset of a
 //    device it has run on (they would belong to the destroyed context).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -85,15 +86,41 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // stream like the kernels that read it. The largest table set (48x48 blocks)
 // is 5248 floats; kernel parameters may take up to 32 KB.
 constexpr int kStaticTableFloats = 7168;
+template <int N>
 struct StaticTableBlob {
-  float v[kStaticTableFloats];
+  float v[N];
 };
 
 // dst[0 .. n) = blob, then dst[n .. n + zeros) = 0 (the unused pattern tables)
-__global__ void k_static_tables(const __grid_constant__ StaticTableBlob b, int n, int zeros, float* dst) {
+template <int N>
+__global__ void k_static_tables(const __grid_constant__ StaticTableBlob<N> b, int n, int zeros, float* dst) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n + zeros; i += gridDim.x * blockDim.x)
     dst[i] = i < n ? b.v[i] : 0.f;
 }
+
+// The tables of blocks up to 32 x 32 (2432 floats) go up in 10 KB of launch
+// parameters, larger ones in 28 KB: the launch copies the whole struct.
+template <int N>
+cudaError_t upload_tables(const std::vector<float>& blob, int zeros, float* dst, cudaStream_t st) {
+  StaticTableBlob<N> tb;
+  std::memcpy(tb.v, blob.data(), blob.size() * sizeof(float));
+  k_static_tables<N><<<8, 256, 0, st>>>(tb, (int)blob.size(), zeros, dst);
+  return cudaGetLastError();
+}
+constexpr int kSmallTableFloats = 2560;
+
+// cos and sin of -2 pi j / n for j < n: a DFT of length n needs no others
+// (k x is taken modulo n)
+struct Roots {
+  std::vector<double> c, s;
+  explicit Roots(int n) : c(n), s(n) {
+    for (int j = 0; j < n; j++) {
+      const double a = -2.0 * M_PI * (double)j / n;
+      c[j] = std::cos(a);
+      s[j] = std::sin(a);
+    }
+  }
+};
 
 }  // namespace
 
@@ -160,19 +187,20 @@ extern "C" int fft3d_filter2d_static(const fft3d_params* p0, const fft3d_plane_d
   {
     const double maxv = bytes == 1 ? 255.0 : (bytes == 2 ? (double)((1 << d->bits) - 1) : 1.0);
     std::vector<double> xr(nh), xi(nh), yr(bh), yi(bh);
+    const Roots rx(bw), ry(bh);
     for (int k = 0; k < nh; k++) {
       double sr = 0, si = 0;
-      for (int x = 0; x < bw; x++) {
-        double a = -2.0 * M_PI * (double)((long)k * x % bw) / bw;
-        sr += wx[x] * std::cos(a); si += wx[x] * std::sin(a);
+      for (int x = 0, j = 0; x < bw; x++) {  // j = k x mod bw
+        sr += wx[x] * rx.c[j]; si += wx[x] * rx.s[j];
+        if ((j += k) >= bw) j -= bw;
       }
       xr[k] = sr; xi[k] = si;
     }
     for (int h = 0; h < bh; h++) {
       double sr = 0, si = 0;
-      for (int y = 0; y < bh; y++) {
-        double a = -2.0 * M_PI * (double)((long)h * y % bh) / bh;
-        sr += wy[y] * std::cos(a); si += wy[y] * std::sin(a);
+      for (int y = 0, j = 0; y < bh; y++) {
+        sr += wy[y] * ry.c[j]; si += wy[y] * ry.s[j];
+        if ((j += h) >= bh) j -= bh;
       }
       yr[h] = sr; yi[h] = si;
     }
@@ -181,19 +209,28 @@ extern "C" int fft3d_filter2d_static(const fft3d_params* p0, const fft3d_plane_d
         grid[2 * (h * nh + k)] = (float)(maxv * (yr[h] * xr[k] - yi[h] * xi[k]));
         grid[2 * (h * nh + k) + 1] = (float)(maxv * (yr[h] * xi[k] + yi[h] * xr[k]));
       }
+    // sharpen and dehalo weights, where the filter reads them; rows j and bh - j are alike
+    const bool sharpen = ep.sharpen != 0, dehalo = ep.dehalo != 0;
     float wmax = 0;
     for (int j = 0; j < bh; j++) {
       int dj = j >= bh / 2 ? bh - j : j;
+      if (dj < j) {
+        std::copy_n(wsh.begin() + dj * nh, nh, wsh.begin() + j * nh);
+        std::copy_n(wdh.begin() + dj * nh, nh, wdh.begin() + j * nh);
+        continue;
+      }
       float d2v = float(dj * dj) * (ep.svr * ep.svr) / ((bh / 2) * (bh / 2));
       for (int i = 0; i < nh; i++) {
         float d2 = d2v + float(i * i) / ((bw / 2) * (bw / 2));
-        wsh[j * nh + i] = (float)(1 - std::exp((double)(-d2 / (2 * ep.scutoff * ep.scutoff))));
+        if (sharpen) wsh[j * nh + i] = (float)(1 - std::exp((double)(-d2 / (2 * ep.scutoff * ep.scutoff))));
+        if (!dehalo) continue;
         float dh = (float)(std::exp((double)(-0.7f * d2 * ep.hr * ep.hr)) - std::exp((double)(-d2 * ep.hr * ep.hr)));
         wdh[j * nh + i] = dh;
         if (dh > wmax) wmax = dh;
       }
     }
-    for (auto& v : wdh) v /= wmax;
+    if (dehalo)
+      for (auto& v : wdh) v /= wmax;
   }
   // scratch layout: tables | spectrum | time-domain blocks
   std::vector<float> blob;
@@ -225,10 +262,9 @@ extern "C" int fft3d_filter2d_static(const fft3d_params* p0, const fft3d_plane_d
   cudaStream_t st = (cudaStream_t)stream;
   char* B = static_cast<char*>(base);
   {
-    StaticTableBlob tb;
-    std::memcpy(tb.v, blob.data(), blob.size() * sizeof(float));
-    k_static_tables<<<8, 256, 0, st>>>(tb, (int)blob.size(), nb, reinterpret_cast<float*>(B));
-    err = cudaGetLastError();
+    float* dst_tables = reinterpret_cast<float*>(B);
+    err = blob.size() <= (size_t)kSmallTableFloats ? upload_tables<kSmallTableFloats>(blob, nb, dst_tables, st)
+                                                   : upload_tables<kStaticTableFloats>(blob, nb, dst_tables, st);
     if (err != cudaSuccess)
       return sfail(FFT3D_E_CUDA, std::string("neo_fft3d: table upload: ") + cudaGetErrorString(err));
   }
