@@ -188,7 +188,7 @@ struct fft3d_plane {
   //   split:   k_forward (new frame), k_filter_bins (streaming filter of all
   //            bins into d_filt), k_filter_inverse<sharpen only> on d_filt
   //   unfused: k_forward, k_filter_inverse (filter + sharpen + inverse)
-  //   fused:   k_fused (new frame's forward + filter + inverse in one launch)
+  //   fused:   k_frame (new frame's forward + filter + inverse in one launch)
   //   tc:      as unfused, with the forward transform on the tensor cores
   //            (k_forward_tc, 32x32 blocks; other sizes fall back to k_forward)
   int path = 1;  // 0 split, 1 unfused, 2 fused, 3 tc
@@ -591,12 +591,66 @@ int copy_plane(fft3d_plane* P, void* dst, int dstride, const void* src, int sstr
   return FFT3D_OK;
 }
 
+// The overlap-add of time-domain blocks `tdom` into the plane at odst.
+fft3d::OlaArgs ola_args(const fft3d_plane* P, const float* tdom, const fft3d::Tables& tab, float base, void* odst,
+                        long long ostride) {
+  fft3d::OlaArgs oa;
+  oa.g = P->g;
+  oa.t = tab;
+  oa.tdom = tdom;
+  oa.dst = static_cast<char*>(odst) + (long long)P->t * ostride + (long long)P->l * P->bytes;
+  oa.dst_stride = ostride;
+  oa.norm = P->norm;
+  const bool ints = P->bytes != 4;
+  oa.rounder = ints ? 0.5f : 0.f;
+  oa.base = base;
+  // float samples clamp to [0, 1] and have no integer maximum (no shift by 32)
+  oa.maxval = P->bytes == 1 ? 255 : (P->bytes == 2 ? (1 << P->d.bits) - 1 : 0);
+  oa.err = P->d_err;
+  return oa;
+}
+
+// The arrival counters of overlap-adds done by the launch that makes their
+// blocks, and the launch's epoch: false when the plane's output tiles are not
+// inside its block grid or the counters cannot be had.
+bool next_ola_epoch(fft3d_plane* P, fft3d::OlaFuse* of, cudaStream_t st) {
+  const fft3d::Geom& g = P->g;
+  of->tiles_x = (g.sx + g.W - 1) / g.sx;
+  of->tiles_y = (g.sy + g.H - 1) / g.sy;
+  if (of->tiles_x < 1 || of->tiles_y < 1 || of->tiles_x >= g.nox || of->tiles_y >= g.noy) return false;
+  const size_t cnt_bytes = (size_t)g.nblocks * sizeof(unsigned);
+  if (!P->d_ola_cnt) {
+    if (dmalloc(P, &P->d_ola_cnt, cnt_bytes) != cudaSuccess) {
+      cudaGetLastError();
+      P->d_ola_cnt = nullptr;
+      return false;
+    }
+    if (cudaMemsetAsync(P->d_ola_cnt, 0, cnt_bytes, st) != cudaSuccess) {
+      cudaGetLastError();
+      dfree(P, P->d_ola_cnt, cnt_bytes);
+      P->d_ola_cnt = nullptr;
+      return false;
+    }
+    P->ola_epoch = 0;
+  }
+  if (P->ola_epoch >= (1u << 29)) {  // targets stay below 2^32: start the counts over
+    if (cudaMemsetAsync(P->d_ola_cnt, 0, cnt_bytes, st) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    P->ola_epoch = 0;
+  }
+  of->cnt = P->d_ola_cnt;
+  of->epoch = ++P->ola_epoch;
+  return true;
+}
+
 // The output of one frame from its time-domain blocks: the crop borders from
 // the source frame (src/fft3d.hpp:292-352), the overlap-add with the tables'
 // synthesis windows and sample offset `base`, and on the host path the
 // download of the result on its own stream.
 int output_frame(fft3d_plane* P, float* tdom, const fft3d::Tables& tab, float base, void* dst, int dst_stride,
-                 const void* cur, int cur_stride, bool host, bool learned, cudaStream_t st) {
+                 const void* cur, int cur_stride, bool host, bool learned, cudaStream_t st, bool ola_done = false) {
   const fft3d_params& ep = P->ep;
   const bool crop = ep.l > 0 || ep.t > 0 || ep.r > 0 || ep.b > 0;
   void* odst = dst;
@@ -617,20 +671,10 @@ int output_frame(fft3d_plane* P, float* tdom, const fft3d::Tables& tab, float ba
     int rc = copy_plane(P, dst, dst_stride, cur, cur_stride, cudaMemcpyDeviceToDevice, st, true);
     if (rc) return rc;
   }
-  fft3d::OlaArgs oa;
-  oa.g = P->g;
-  oa.t = tab;
-  oa.tdom = tdom;
-  oa.dst = static_cast<char*>(odst) + (long long)P->t * ostride + (long long)P->l * P->bytes;
-  oa.dst_stride = ostride;
-  oa.norm = P->norm;
-  const bool ints = P->bytes != 4;
-  oa.rounder = ints ? 0.5f : 0.f;
-  oa.base = base;
-  // float samples clamp to [0, 1] and have no integer maximum (no shift by 32)
-  oa.maxval = P->bytes == 1 ? 255 : (P->bytes == 2 ? (1 << P->d.bits) - 1 : 0);
-  oa.err = P->d_err;
-  if (g_defer) {
+  fft3d::OlaArgs oa = ola_args(P, tdom, tab, base, odst, ostride);
+  if (ola_done) {
+    // the frame's launch did it
+  } else if (g_defer) {
     g_defer->ola.push_back({oa, P->bytes, g_defer->plane});
   } else {
     TimeScope ts(P, K_OLA, (double)P->g.nblocks * P->g.bh * P->g.bw * 4 + (double)P->g.W * P->g.H * P->bytes, st);
@@ -777,6 +821,9 @@ int pshow_frame(fft3d_plane* P, int n, const void* const src[5], const int strid
   return output_frame(P, P->d_tdom, tab, base, dst, dst_stride, cur, stride[2], host, false, st);
 }
 
+// Most blocks of a plane whose frames go in one launch (k_frame).
+constexpr int kOneLaunchBlocks = 600;
+
 int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride[5], void* dst, int dst_stride,
                bool host, cudaStream_t st) {
   if (P->reset_pending) {  // fft3d_plane_reset queued on the plane's stream
@@ -818,7 +865,11 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
   // of the window, in the fused kernel; older frames missing from the ring
   // (clip start, seeks) are transformed first by the forward kernel.
   const int newest = n + to;
-  const bool fused = P->path == 2 && P->bytes != 4 && !learned && !find_slot(P, newest);
+  // Small planes (device calls, one frame at a time) do the whole frame in one
+  // launch, the overlap-add too.
+  const bool small = P->path == 1 && !host && !g_defer && !P->bulk && P->g.nblocks <= kOneLaunchBlocks;
+  const bool fused = (P->path == 2 || small) && P->bytes != 4 && !learned && !find_slot(P, newest);
+  bool ola_done = false;
   for (int d = from; d <= (fused ? to - 1 : to); d++) {
     Slot* s = nullptr;
     int rc = spectrum_slot(P, n + d, n + from, n + to, src ? src[2 + d] : nullptr, stride ? stride[2 + d] : 0, host,
@@ -890,12 +941,28 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
     if (fused) {
       // reads: the newest frame's pixels and the older spectra (+ Kalman state);
       // writes: the newest spectrum and the time-domain blocks
-      fft3d::FusedArgs fa;
+      fft3d::FrameArgs fa;
       fa.f = forward_args(P, new_src, new_stride, news->spec);
       fa.v = ia;
+      fa.of = fft3d::OlaFuse{};
+      if (small && next_ola_epoch(P, &fa.of, st)) {
+        fa.of.o = ola_args(P, nullptr, P->tab, fa.f.base, dst, dst_stride);
+        fft3d::OlaFrameSet fs{};
+        fs.count = 1;
+        fs.tdom[0] = tdom;
+        fa.of.dst[0] = fs.dst[0] = fa.of.o.dst;
+        fa.of.dst_stride[0] = fs.dst_stride[0] = dst_stride;
+        fa.of.bytes = P->bytes;
+        fa.of.px4 = fft3d::overlap_add_frames_supported(fa.of.o, fs, P->bytes) ? 1 : 0;
+        fa.of.o.dst = nullptr;
+        ola_done = true;
+      }
       {
-        TimeScope ts(P, K_FUSED, (double)P->g.W * P->g.H * P->bytes + (to - from) * S + S + state + T, st);
-        CK(fft3d::launch_fused(fa, mode, P->bytes, st), "fused kernel");
+        const double pix = (double)P->g.W * P->g.H * P->bytes;
+        TimeScope ts(P, K_FUSED, pix + (to - from) * S + S + state + (ola_done ? pix : T), st);
+        const cudaError_t le = fft3d::launch_frame(fa, mode, P->bytes, st);
+        if (le != cudaSuccess && ola_done) P->ola_epoch--;  // no arrivals were counted for this epoch
+        CK(le, "one-launch kernel");
       }
       if (host) CK(cudaEventRecord(P->cur->in_free, st), "event");
     } else if (P->path == 0 && mode != fft3d::MODE_SHARPEN_ONLY) {
@@ -926,7 +993,7 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
   if (!g_defer) g_launches++;
   const bool ints = P->bytes != 4;
   return output_frame(P, tdom, P->tab, (ints && P->d.is_chroma) ? (float)(1 << (P->d.bits - 1)) : 0.f, dst,
-                      dst_stride, cur, stride ? stride[2] : 0, host, learned, st);
+                      dst_stride, cur, stride ? stride[2] : 0, host, learned, st, ola_done);
 }
 
 // A stage for one host-path call, exclusive until the call returns (the
@@ -1050,9 +1117,6 @@ void discard_recorded(fft3d_plane* P, const fft3d::Deferred& d) {
 bool fuse_run_ola(fft3d_plane* P, const fft3d::Deferred& d, const fft3d::TemporalSet& ts, size_t i, size_t e,
                   std::vector<char>& ola_done, fft3d::OlaFuse* of, cudaStream_t st) {
   if (!P->fuse_ola || e - i > (size_t)fft3d::kGroupTile) return false;
-  const fft3d::Geom& g = P->g;
-  const int tiles_x = (g.sx + g.W - 1) / g.sx, tiles_y = (g.sy + g.H - 1) / g.sy;
-  if (tiles_x < 1 || tiles_y < 1 || tiles_x >= g.nox || tiles_y >= g.noy) return false;
   size_t idx[fft3d::kGroupTile];
   for (size_t k = i; k < e; k++) {
     size_t m = 0;
@@ -1060,30 +1124,8 @@ bool fuse_run_ola(fft3d_plane* P, const fft3d::Deferred& d, const fft3d::Tempora
     if (m == d.ola.size() || (k > i && d.ola[m].bytes != d.ola[idx[0]].bytes)) return false;
     idx[k - i] = m;
   }
-  const size_t cnt_bytes = (size_t)g.nblocks * sizeof(unsigned);
-  if (!P->d_ola_cnt) {
-    if (dmalloc(P, &P->d_ola_cnt, cnt_bytes) != cudaSuccess) {
-      cudaGetLastError();
-      P->d_ola_cnt = nullptr;
-      return false;
-    }
-    if (cudaMemsetAsync(P->d_ola_cnt, 0, cnt_bytes, st) != cudaSuccess) {
-      cudaGetLastError();
-      cudaFree(P->d_ola_cnt);
-      P->d_ola_cnt = nullptr;
-      return false;
-    }
-    P->ola_epoch = 0;
-  }
-  if (P->ola_epoch >= (1u << 29)) {  // targets stay below 2^32: start the counts over
-    if (cudaMemsetAsync(P->d_ola_cnt, 0, cnt_bytes, st) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    P->ola_epoch = 0;
-  }
-  P->ola_epoch++;
   *of = fft3d::OlaFuse{};
+  if (!next_ola_epoch(P, of, st)) return false;
   of->o = d.ola[idx[0]].a;
   of->o.tdom = nullptr;
   of->o.dst = nullptr;
@@ -1097,10 +1139,6 @@ bool fuse_run_ola(fft3d_plane* P, const fft3d::Deferred& d, const fft3d::Tempora
     fs.dst_stride[k] = of->dst_stride[k];
     ola_done[idx[k]] = 1;
   }
-  of->cnt = P->d_ola_cnt;
-  of->epoch = P->ola_epoch;
-  of->tiles_x = tiles_x;
-  of->tiles_y = tiles_y;
   of->bytes = d.ola[idx[0]].bytes;
   of->px4 = fft3d::overlap_add_frames_supported(of->o, fs, of->bytes) ? 1 : 0;
   return true;

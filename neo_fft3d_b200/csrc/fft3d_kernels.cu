@@ -286,9 +286,9 @@ cudaError_t launch_filter_frames(const InverseArgs& a, const FilterFrameSet& fs,
   return cudaGetLastError();
 }
 
-cudaError_t launch_fused(const FusedArgs& a, int mode, int bytes, cudaStream_t s) {
+cudaError_t launch_frame(const FrameArgs& a, int mode, int bytes, cudaStream_t s) {
   const SizeEntry* e = find_size(a.v.g.bw, a.v.g.bh);
-  return e ? e->fused(a, mode, bytes, s) : cudaErrorInvalidValue;
+  return e ? e->frame(a, mode, bytes, s) : cudaErrorInvalidValue;
 }
 
 cudaError_t launch_forward_batch(int bw, int bh, const BatchLaunch& l, int bytes, cudaStream_t s) {

@@ -186,14 +186,6 @@ struct OlaFrameSet {
   int count;
 };
 
-// Forward transform of the window's newest frame fused with the filter and
-// the inverse transform (k_fused). f.src/f.spec: the newest frame and its ring
-// slot; v.in[]: the window's spectra (the newest frame's entry is f.spec).
-struct FusedArgs {
-  ForwardArgs f;
-  InverseArgs v;
-};
-
 struct OlaArgs {
   Geom g;
   Tables t;
@@ -225,6 +217,16 @@ struct OlaFuse {
   int tiles_x, tiles_y;
   int bytes;                      // sample size: 1, 2 or 4
   int px4;                        // 4-pixel form (the plane meets its rules)
+};
+
+// One output frame in one launch (k_frame). f.src/f.spec: the window's newest
+// frame and its ring slot; v.in[]: the window's spectra (the newest frame's
+// entry is f.spec); of: the overlap-add's arguments where the same launch does
+// it (of.cnt set), as for a run of one frame.
+struct FrameArgs {
+  ForwardArgs f;
+  InverseArgs v;
+  OlaFuse of;
 };
 
 // One batched launch: `nitems` work items (plane index into `args`, CTA of
@@ -304,8 +306,8 @@ cudaError_t launch_filter_bins(const InverseArgs& a, float2* F, int mode, cudaSt
 // MODE_SHARPEN_ONLY on fs.out). Kalman runs walk the frames in order, with
 // the state in registers from the run's first frame to its last.
 cudaError_t launch_filter_frames(const InverseArgs& a, const FilterFrameSet& fs, int mode, cudaStream_t s);
-// cudaErrorNotSupported when no fused kernel exists for the sample type (float)
-cudaError_t launch_fused(const FusedArgs& a, int mode, int bytes_per_sample, cudaStream_t s);
+// cudaErrorNotSupported when no one-launch kernel exists for the sample type (float)
+cudaError_t launch_frame(const FrameArgs& a, int mode, int bytes_per_sample, cudaStream_t s);
 bool block_size_supported(int bw, int bh);
 // FindPatternBlock scores (src/helper.cpp:46-90): scores[(by-2)*(nox-4) + bx-2] =
 // sum over bins of |X - gridfraction * grid|^2 * pwin for the interior blocks

@@ -106,35 +106,43 @@ __host__ __device__ constexpr int fft_smem_bytes() {
   return blocks_per_warp<BW>() * BH * (BW / 2 + 1) * 8;
 }
 
-// Row of BW samples starting at p, as floats; 16-byte vector loads when the
-// row is aligned (the common interior case), scalar loads otherwise.
+// The BW samples at p as 32-bit words: 16-byte loads where p allows, else
+// 4-byte loads of the words that hold them (never past the word of the last
+// sample) and funnel shifts.
 template <typename T, int BW>
-__device__ __forceinline__ void load_row(const T* p, float (&r)[BW]) {
-  constexpr int BYTES = BW * (int)sizeof(T);
-  if constexpr (BYTES % 16 == 0) {
-    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-      const uint4* q = reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void load_words(const T* p, uint32_t (&w)[BW * sizeof(T) / 4]) {
+  constexpr int WORDS = BW * (int)sizeof(T) / 4;
+  static_assert(BW * sizeof(T) % 4 == 0, "whole words");
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  if (WORDS % 4 == 0 && (at & 15) == 0) {
+    const uint4* q = reinterpret_cast<const uint4*>(p);
 #pragma unroll
-      for (int v = 0; v < BYTES / 16; v++) {
-        const uint4 u = __ldg(q + v);
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-        constexpr int PER = 16 / (int)sizeof(T);
+    for (int v = 0; v < WORDS / 4; v++) {
+      const uint4 u = __ldg(q + v);
+      w[4 * v] = u.x, w[4 * v + 1] = u.y, w[4 * v + 2] = u.z, w[4 * v + 3] = u.w;
+    }
+    return;
+  }
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(at & ~(uintptr_t)3);
 #pragma unroll
-        for (int j = 0; j < PER; j++) {
-          float f;  // 8/16-bit: exact through the 2^23 mantissa trick (decode_row)
-          if constexpr (sizeof(T) == 1)
-            f = __uint_as_float(__byte_perm(w[j >> 2], 0x4B000000u, 0x7540u | (uint32_t)(j & 3))) - 8388608.0f;
-          else if constexpr (sizeof(T) == 2)
-            f = __uint_as_float(__byte_perm(w[j >> 1], 0x4B000000u, (j & 1) ? 0x7432u : 0x7410u)) - 8388608.0f;
-          else f = __uint_as_float(w[j]);
-          r[v * PER + j] = f;
-        }
-      }
-      return;
+  for (int v = 0; v < WORDS; v++) w[v] = __ldg(q + v);
+  if constexpr (sizeof(T) < 4) {
+    const int shift = 8 * (int)(at & 3);
+    if (shift) {
+      const uint32_t last = __ldg(q + WORDS);
+#pragma unroll
+      for (int v = 0; v < WORDS; v++) w[v] = __funnelshift_r(w[v], v + 1 < WORDS ? w[v + 1] : last, shift);
     }
   }
-#pragma unroll
-  for (int x = 0; x < BW; x++) r[x] = load_sample<T>(p + x);
+}
+
+// Sample x of a row's words as a float of 2^23 + sample (8/16-bit samples: one
+// byte permute into the low mantissa bits of 2^23, exact), or the sample itself.
+template <typename T, int WORDS>
+__device__ __forceinline__ float raw_sample(const uint32_t (&w)[WORDS], int x) {
+  if constexpr (sizeof(T) == 1) return __uint_as_float(__byte_perm(w[x >> 2], 0x4B000000u, 0x7540u | (uint32_t)(x & 3)));
+  else if constexpr (sizeof(T) == 2) return __uint_as_float(__byte_perm(w[x >> 1], 0x4B000000u, (x & 1) ? 0x7432u : 0x7410u));
+  else return __uint_as_float(w[x]);
 }
 
 // ---------------------------------------------------------------- block FFT phases
@@ -182,18 +190,22 @@ __device__ __forceinline__ void fwd_row(const ForwardArgs& a, const Win& win, in
   const T* srow = fwd_row_src<T>(a, win, blk, y, &x0, &srcrow);
   float r[BW];
   const bool row_ok = FFT3D_IN(srcrow >= 0 && srcrow < g.H, a.err);
-  if (x0 >= 0 && x0 + BW <= g.W) {
-    if (row_ok) load_row<T, BW>(srow + x0, r);
+  const float off = (sizeof(T) < 4 ? 8388608.0f : 0.f) + a.base;  // raw_sample's offset and the plane's: exact
+  if (row_ok && x0 >= 0 && x0 + BW <= g.W) {
+    uint32_t w[BW * sizeof(T) / 4];
+    load_words<T, BW>(srow + x0, w);
+#pragma unroll
+    for (int x = 0; x < BW; x++) r[x] = raw_sample<T>(w, x) - off;
   } else {
 #pragma unroll
     for (int x = 0; x < BW; x++) {
       const int xi = reflect101(x0 + x, g.W);
-      r[x] = (row_ok && FFT3D_IN(xi >= 0 && xi < g.W, a.err)) ? load_sample<T>(srow + xi) : 0.f;
+      r[x] = (row_ok && FFT3D_IN(xi >= 0 && xi < g.W, a.err)) ? load_sample<T>(srow + xi) - a.base : 0.f;
     }
   }
   const float wy = __ldg(a.wan_y + y);
 #pragma unroll
-  for (int x = 0; x < BW; x++) r[x] = (r[x] - a.base) * __ldg(a.wan_x + x) * wy;
+  for (int x = 0; x < BW; x++) r[x] = r[x] * __ldg(a.wan_x + x) * wy;
   float2 c[NH];
   rfft<BW>(r, c);
   float2* row = Sb + y * NH;
@@ -290,36 +302,28 @@ __device__ __forceinline__ void store_tdom(const float2* Sb, float* out, int lan
 
 // ---------------------------------------------------------------- forward
 
-// k_fused's forward part: one warp transforms blocks_per_warp<BW>()
-// consecutive blocks (rows, then columns, then a coalesced 16-byte copy-out of
-// the contiguous spectra), which stay in the warp's shared memory.
+// k_frame's forward part: the CTA transforms `count` consecutive blocks into
+// the tiles at S (a row, then a column per thread) and copies them to the
+// ring; the tiles stay for the filter. The caller's next barrier ends the copy.
 template <int BW, int BH, typename T>
-__device__ __forceinline__ void forward_cta(const ForwardArgs& a, int cta) {
-  constexpr int NH = BW / 2 + 1, HC = BW / 2, NBW = blocks_per_warp<BW>(), BINS = BH * NH;
-  extern __shared__ __align__(16) float2 smem2[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float2* S = smem2 + warp * NBW * BINS;
-  const Geom& g = a.g;
+__device__ __forceinline__ void frame_forward(const ForwardArgs& a, int blk0, int count, float2* S) {
+  constexpr int NH = BW / 2 + 1, HC = BW / 2, BINS = BH * NH, NT = kWarps * 32;
   const ArgsFwd win{a};
-  const int blk0 = (cta * kWarps + warp) * NBW;
-  if (blk0 >= g.nblocks) return;
-  for (int t = lane; t < NBW * BH; t += 32) {
-    const int b = t / BH, y = t - b * BH;
-    if (blk0 + b < g.nblocks) fwd_row<BW, BH, T>(a, win, blk0 + b, y, S + b * BINS);
+  const int t = threadIdx.x;
+  for (int i = t; i < count * BH; i += NT) {
+    const int b = i / BH;
+    fwd_row<BW, BH, T>(a, win, blk0 + b, i - b * BH, S + b * BINS);
   }
-  __syncwarp();
-  for (int t = lane; t < NBW * HC; t += 32) {
-    const int b = t / HC, c = t - b * HC;
-    if (blk0 + b < g.nblocks) fwd_col<BW, BH>(S + b * BINS, c);
+  __syncthreads();
+  for (int i = t; i < count * HC; i += NT) {
+    const int b = i / HC;
+    fwd_col<BW, BH>(S + b * BINS, i - b * HC);
   }
-  __syncwarp();
-  const int nvalid = min(NBW, g.nblocks - blk0);
-  float4* dst = reinterpret_cast<float4*>(win.spec() + (size_t)blk0 * BINS);
+  __syncthreads();
+  float4* dst = reinterpret_cast<float4*>(a.spec + (size_t)blk0 * BINS);
   const float4* src = reinterpret_cast<const float4*>(S);
-  for (int i = lane; i < nvalid * BINS / 2; i += 32)
-    if (FFT3D_IN((size_t)blk0 * BINS / 2 + i < (size_t)g.nblocks * BINS / 2 && win.spec() != nullptr, a.err))
-      dst[i] = src[i];
-  __syncwarp();
+  for (int i = t; i < count * BINS / 2; i += NT)
+    if (FFT3D_IN((size_t)blk0 * BINS / 2 + i < (size_t)a.g.nblocks * BINS / 2 && a.spec != nullptr, a.err)) dst[i] = src[i];
 }
 
 // Blocks of a forward CTA, and its threads: one per column (DC and Nyquist
@@ -330,45 +334,6 @@ template <int BW>
 __host__ __device__ constexpr int fwd_blocks() { return kWarps * blocks_per_warp<BW>(); }
 template <int BW>
 __host__ __device__ constexpr int fwd_threads() { return fwd_blocks<BW>() * (BW / 2); }
-
-// The BW samples at p as 32-bit words: 16-byte loads where p allows, else
-// 4-byte loads of the words that hold them (never past the word of the last
-// sample) and funnel shifts.
-template <typename T, int BW>
-__device__ __forceinline__ void load_words(const T* p, uint32_t (&w)[BW * sizeof(T) / 4]) {
-  constexpr int WORDS = BW * (int)sizeof(T) / 4;
-  static_assert(BW * sizeof(T) % 4 == 0, "whole words");
-  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
-  if (WORDS % 4 == 0 && (at & 15) == 0) {
-    const uint4* q = reinterpret_cast<const uint4*>(p);
-#pragma unroll
-    for (int v = 0; v < WORDS / 4; v++) {
-      const uint4 u = __ldg(q + v);
-      w[4 * v] = u.x, w[4 * v + 1] = u.y, w[4 * v + 2] = u.z, w[4 * v + 3] = u.w;
-    }
-    return;
-  }
-  const uint32_t* q = reinterpret_cast<const uint32_t*>(at & ~(uintptr_t)3);
-#pragma unroll
-  for (int v = 0; v < WORDS; v++) w[v] = __ldg(q + v);
-  if constexpr (sizeof(T) < 4) {
-    const int shift = 8 * (int)(at & 3);
-    if (shift) {
-      const uint32_t last = __ldg(q + WORDS);
-#pragma unroll
-      for (int v = 0; v < WORDS; v++) w[v] = __funnelshift_r(w[v], v + 1 < WORDS ? w[v + 1] : last, shift);
-    }
-  }
-}
-
-// Sample x of a row's words as a float of 2^23 + sample (8/16-bit samples: one
-// byte permute into the low mantissa bits of 2^23, exact), or the sample itself.
-template <typename T, int WORDS>
-__device__ __forceinline__ float raw_sample(const uint32_t (&w)[WORDS], int x) {
-  if constexpr (sizeof(T) == 1) return __uint_as_float(__byte_perm(w[x >> 2], 0x4B000000u, 0x7540u | (uint32_t)(x & 3)));
-  else if constexpr (sizeof(T) == 2) return __uint_as_float(__byte_perm(w[x >> 1], 0x4B000000u, (x & 1) ? 0x7432u : 0x7410u));
-  else return __uint_as_float(w[x]);
-}
 
 // Forward transform of fwd_blocks<BW>() consecutive blocks per CTA.
 //  rows: a thread takes rows y and y + bh/2 of a block at once, packed
@@ -1069,9 +1034,7 @@ struct FrameWin {
   __device__ __forceinline__ float* tdom() const { return t; }
 };
 
-// NEWEST_IN_S: the window's newest frame (slot win_hi) is not read from
-// the window but from S, where the fused kernel's forward transform left it.
-template <int BW, int BH, int MODE, bool NEWEST_IN_S, class Win>
+template <int BW, int BH, int MODE, class Win>
 __device__ __forceinline__ void filter_inverse_cta_w(const InverseArgs& a, int vcta, const Win& win) {
   constexpr int NH = BW / 2 + 1, HC = BW / 2, NBW = blocks_per_warp<BW>(), BINS = BH * NH;
   constexpr int PER = (BINS / 2 + 31) / 32;
@@ -1084,11 +1047,9 @@ __device__ __forceinline__ void filter_inverse_cta_w(const InverseArgs& a, int v
   if (blk0 >= g.nblocks) return;
   const float gs0 = __ldg(&a.t.grid[0].x);
   constexpr int LO = win_lo<MODE>(), HI = win_hi<MODE>(), NW = HI - LO + 1;
-  constexpr int NG = NEWEST_IN_S ? NW - 1 : NW;  // window slots read from global memory
-  constexpr int NGB = NG > 0 ? NG : 1;
   // load-pipeline depth (chunks of 32 bin pairs in flight), fewer as the
   // window (and the registers per chunk) grows
-  constexpr int DW = NG <= 1 ? 4 : (NG == 2 ? 4 : (NG == 3 ? 3 : 2));
+  constexpr int DW = NW <= 1 ? 4 : (NW == 2 ? 4 : (NW == 3 ? 3 : 2));
   constexpr int D = PER < DW ? PER : DW;
 #pragma unroll 1
   for (int b = 0; b < NBW; b++) {
@@ -1096,29 +1057,20 @@ __device__ __forceinline__ void filter_inverse_cta_w(const InverseArgs& a, int v
     if (blk >= g.nblocks) break;
     const size_t off = (size_t)blk * BINS;
     float gf = 0.f;
-    if constexpr (MODE >= 1) {
-      if (NEWEST_IN_S && HI == 2) {
-        gf = a.c.degrid * S[b * BINS].x / gs0;
-        __syncwarp();  // every lane has the DC before lane 0 overwrites it
-      } else {
-        gf = a.c.degrid * __ldg(&win.in(2)[off].x) / gs0;
-      }
-    }
+    if constexpr (MODE >= 1) gf = a.c.degrid * __ldg(&win.in(2)[off].x) / gs0;
     // software pipeline: the window's values of chunk j + D are loaded while
-    // chunk j is filtered, so D x NG loads per lane are always in flight
-    float4 buf[D][NGB];
-    auto load = [&](int j, float4(&dst)[NGB]) {
+    // chunk j is filtered, so D x NW loads per lane are always in flight
+    float4 buf[D][NW];
+    auto load = [&](int j, float4(&dst)[NW]) {
       const int i = 2 * (lane + 32 * j);
 #pragma unroll
-      for (int k = 0; k < NG; k++)
+      for (int k = 0; k < NW; k++)
         dst[k] = (i < BINS && FFT3D_IN(win.in(LO + k) != nullptr && off + i + 1 < (size_t)g.nblocks * BINS, a.err))
                      ? ld_stream4(win.in(LO + k) + off + i)
                      : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    if constexpr (NG > 0) {
 #pragma unroll
-      for (int j = 0; j < D; j++) load(j, buf[j]);
-    }
+    for (int j = 0; j < D; j++) load(j, buf[j]);
     float gsh = 0.f;
     // (D chunks to a turn of the loop: the whole block unrolled is four times
     // the code, and its instruction-cache misses cost more than the loop)
@@ -1131,9 +1083,8 @@ __device__ __forceinline__ void filter_inverse_cta_w(const InverseArgs& a, int v
         const bool in = i < BINS;
         float4 w[5];
 #pragma unroll
-        for (int k = 0; k < 5; k++) w[k] = (k >= LO && k < LO + NG) ? buf[u][k - LO] : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (NEWEST_IN_S && in) w[HI] = *reinterpret_cast<const float4*>(S + b * BINS + i);
-        if (NG > 0 && j + D < PER) load(j + D, buf[u]);
+        for (int k = 0; k < 5; k++) w[k] = (k >= LO && k < LO + NW) ? buf[u][k - LO] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j + D < PER) load(j + D, buf[u]);
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (in) {
           if constexpr (MODE == MODE_KALMAN) {
@@ -1172,9 +1123,9 @@ __device__ __forceinline__ void filter_inverse_cta_w(const InverseArgs& a, int v
   __syncwarp();  // S is reused by the warp's next work item
 }
 
-template <int BW, int BH, int MODE, bool NEWEST_IN_S = false>
+template <int BW, int BH, int MODE>
 __device__ __forceinline__ void filter_inverse_cta(const InverseArgs& a, int vcta) {
-  filter_inverse_cta_w<BW, BH, MODE, NEWEST_IN_S, ArgsWin>(a, vcta, ArgsWin{a});
+  filter_inverse_cta_w<BW, BH, MODE, ArgsWin>(a, vcta, ArgsWin{a});
 }
 
 // Several consecutive output frames of one plane in one launch (a frame
@@ -1199,7 +1150,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_filter_inverse_frames(InverseAr
       for (int k = 0; k < 5; k++) w.p[k] = fs.in[q][k];
       w.t = fs.tdom[q];
     }
-  filter_inverse_cta_w<BW, BH, MODE, false, FrameWin>(a, c, w);
+  filter_inverse_cta_w<BW, BH, MODE, FrameWin>(a, c, w);
 }
 
 template <int BW, int BH, int MODE>
@@ -1661,8 +1612,10 @@ __host__ __device__ constexpr int run_ctas(int extra) {
 //     complex transform), 4. the c2r rows, 5. coalesced stores of the
 //     time-domain blocks.
 // bar: an initialised mbarrier (STAGED), whose parity is `phase`. False when
-// the bounded wait on it ran out (the whole CTA then leaves).
-template <int BW, int BH, int MODE, bool STAGED>
+// the bounded wait on it ran out (the whole CTA then leaves). NEWEST (one
+// frame, not staged): the window's newest spectrum is not read from the window
+// but from the tiles, where k_frame's forward transform left it.
+template <int BW, int BH, int MODE, bool STAGED, bool NEWEST = false>
 __device__ __forceinline__ bool filter_inverse_group_cta(const InverseArgs& a, const TemporalSet& ts, int cta,
                                                          uint64_t* bar, uint32_t phase, const OlaFuse* of = nullptr) {
   constexpr int NH = BW / 2 + 1, HC = BW / 2, BINS = BH * NH, PAIRS = BINS / 2, NT = kWarps * 32;
@@ -1701,6 +1654,7 @@ __device__ __forceinline__ bool filter_inverse_group_cta(const InverseArgs& a, c
   }
   auto load = [&](int s, int b, int bin) {
     if constexpr (STAGED) return *reinterpret_cast<const float4*>(S + ((s - LO) * nbv + b) * BINS + bin);
+    else if (NEWEST && s == HI) return *reinterpret_cast<const float4*>(S + b * BINS + bin);
     else return group_load(a, ts, s, off0 + b * BINS, bin);
   };
   constexpr bool WALK = MODE == MODE_KALMAN || MODE >= 2;
@@ -1763,6 +1717,8 @@ __device__ __forceinline__ bool filter_inverse_group_cta(const InverseArgs& a, c
       bulk_wait(bar, phase);
       return false;
     }
+  } else if constexpr (NEWEST) {
+    __syncthreads();  // the tiles' copies to the ring are done
   }
   using Cursor = PairCursor<BINS, NT>;
   if constexpr (WALK) {
@@ -2007,19 +1963,23 @@ __global__ void __launch_bounds__(kBulkWarps * 32) k_filter_inverse_bulk(Inverse
   }
 }
 
-// ---------------------------------------------------------------- fused
+// ---------------------------------------------------------------- one launch per frame
 
-// Steady-state hot path of one output frame in one launch: each warp
-// transforms the window's newest frame for its blocks (forward_cta: the
-// spectra go to the ring for the next output frames and stay in the warp's
-// shared memory), then filters and inverse-transforms them
-// (filter_inverse_cta) with the older frames' spectra streamed from the ring
-// through the same register load pipeline as k_filter_inverse.
+// One output frame in one launch: each CTA transforms the window's newest frame
+// for its blocks (the spectra go to the ring for the next output frames and
+// stay in its tiles), filters them with the older frames' spectra from the
+// ring and inverse-transforms them; with `of`, the CTA that completes an
+// output tile does its overlap-add. For small planes, whose frames cost their
+// launches and the latency of three kernels' chains rather than any
+// throughput.
 template <int BW, int BH, typename T, int MODE>
-__global__ void __launch_bounds__(kWarps * 32, 6) k_fused(FusedArgs A) {
-  const int n = fft_ctas<BW, BH>(A.v.g.nblocks);
-  forward_cta<BW, BH, T>(A.f, A.v.reverse ? n - 1 - (int)blockIdx.x : (int)blockIdx.x);
-  filter_inverse_cta<BW, BH, MODE, true>(A.v, blockIdx.x);
+__global__ void __launch_bounds__(kWarps * 32, 3)
+    k_frame(const __grid_constant__ ForwardArgs f, const __grid_constant__ InverseArgs a,
+            const __grid_constant__ TemporalSet ts, const __grid_constant__ OlaFuse of) {
+  extern __shared__ __align__(16) float2 smem2[];
+  const int blk0 = blockIdx.x * ts.nb;
+  frame_forward<BW, BH, T>(f, blk0, min(ts.nb, a.g.nblocks - blk0), smem2 + group_head_floats<BW, BH>() / 2);
+  filter_inverse_group_cta<BW, BH, MODE, false, true>(a, ts, blockIdx.x, nullptr, 0, of.cnt ? &of : nullptr);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -2128,6 +2088,11 @@ cudaError_t fwd_sized(const ForwardArgs& a, int bytes, cudaStream_t s) {
   return fwd_frames<BW, BH>(a, fs, bytes, s);
 }
 
+inline bool ola_fuse_ok(const OlaFuse& of, const Geom& g) {
+  return of.cnt && of.epoch != 0 && of.tiles_x >= 1 && of.tiles_y >= 1 && of.tiles_x < g.nox && of.tiles_y < g.noy &&
+         (of.bytes == 1 || of.bytes == 2 || of.bytes == 4);
+}
+
 // Blocks per CTA of a run whose block takes `count` tiles, over nblocks
 // blocks: as many as the CTA has tiles for, but no more than keep every CTA
 // slot of the chip filled (6 per SM), down to one block per CTA for small
@@ -2206,34 +2171,38 @@ cudaError_t inv_mode(const InverseArgs& a, cudaStream_t s) {
 }
 
 template <int BW, int BH, typename T, int MODE>
-cudaError_t fused_mode(const FusedArgs& a, cudaStream_t s) {
-  const int smem = kWarps * fft_smem_bytes<BW, BH>();
-  const int grid = fft_ctas<BW, BH>(a.v.g.nblocks);
-  cudaError_t e =
-      fft3d::smem_attr(k_fused<BW, BH, T, MODE>, smem);
+cudaError_t frame_mode(const FrameArgs& a, cudaStream_t s) {
+  cudaError_t e = fft3d::smem_attr(k_frame<BW, BH, T, MODE>, group_smem_bytes<BW, BH>(group_tiles<BW, BH>()));
   if (e != cudaSuccess) return e;
-  k_fused<BW, BH, T, MODE><<<grid, kWarps * 32, smem, s>>>(a);
+  TemporalSet ts{};
+  ts.count = 1;
+  for (int k = 0; k < 5; k++) ts.spec[k] = a.v.in[k];
+  ts.tdom[0] = a.v.tdom;
+  ts.nb = a.of.cnt ? 1 : group_blocks_per_cta<BW, BH, MODE, false>(a.v.g.nblocks, 1);
+  k_frame<BW, BH, T, MODE><<<(a.v.g.nblocks + ts.nb - 1) / ts.nb, kWarps * 32, group_smem_bytes<BW, BH>(ts.nb), s>>>(
+      a.f, a.v, ts, a.of);
   return cudaGetLastError();
 }
 
 template <int BW, int BH, typename T>
-cudaError_t fused_typed(const FusedArgs& a, int mode, cudaStream_t s) {
+cudaError_t frame_typed(const FrameArgs& a, int mode, cudaStream_t s) {
   switch (mode) {
-    case MODE_SHARPEN_ONLY: return fused_mode<BW, BH, T, MODE_SHARPEN_ONLY>(a, s);
-    case MODE_KALMAN: return fused_mode<BW, BH, T, MODE_KALMAN>(a, s);
-    case 1: return fused_mode<BW, BH, T, 1>(a, s);
-    case 2: return fused_mode<BW, BH, T, 2>(a, s);
-    case 3: return fused_mode<BW, BH, T, 3>(a, s);
-    case 4: return fused_mode<BW, BH, T, 4>(a, s);
-    case 5: return fused_mode<BW, BH, T, 5>(a, s);
+    case MODE_SHARPEN_ONLY: return frame_mode<BW, BH, T, MODE_SHARPEN_ONLY>(a, s);
+    case MODE_KALMAN: return frame_mode<BW, BH, T, MODE_KALMAN>(a, s);
+    case 1: return frame_mode<BW, BH, T, 1>(a, s);
+    case 2: return frame_mode<BW, BH, T, 2>(a, s);
+    case 3: return frame_mode<BW, BH, T, 3>(a, s);
+    case 4: return frame_mode<BW, BH, T, 4>(a, s);
+    case 5: return frame_mode<BW, BH, T, 5>(a, s);
   }
   return cudaErrorInvalidValue;
 }
 
 template <int BW, int BH>
-cudaError_t fused_sized(const FusedArgs& a, int mode, int bytes, cudaStream_t s) {
-  if (bytes == 1) return fused_typed<BW, BH, uint8_t>(a, mode, s);
-  if (bytes == 2) return fused_typed<BW, BH, uint16_t>(a, mode, s);
+cudaError_t frame_sized(const FrameArgs& a, int mode, int bytes, cudaStream_t s) {
+  if (a.of.cnt && !ola_fuse_ok(a.of, a.v.g)) return cudaErrorInvalidValue;
+  if (bytes == 1) return frame_typed<BW, BH, uint8_t>(a, mode, s);
+  if (bytes == 2) return frame_typed<BW, BH, uint16_t>(a, mode, s);
   return cudaErrorNotSupported;  // float samples use the unfused path
 }
 
@@ -2267,9 +2236,7 @@ cudaError_t inv_group(const InverseArgs& a, const TemporalSet& ts, int mode, cud
   OlaFuse of{};
   if (ofp) {
     of = *ofp;
-    if (!of.cnt || of.epoch == 0 || of.tiles_x < 1 || of.tiles_y < 1 || of.tiles_x >= a.g.nox ||
-        of.tiles_y >= a.g.noy || (of.bytes != 1 && of.bytes != 2 && of.bytes != 4))
-      return cudaErrorInvalidValue;
+    if (!ola_fuse_ok(of, a.g)) return cudaErrorInvalidValue;
   }
   switch (mode) {
     case MODE_SHARPEN_ONLY: return inv_group_mode<BW, BH, MODE_SHARPEN_ONLY>(a, ts, of, s);
@@ -2326,7 +2293,7 @@ cudaError_t inv_sized(const InverseArgs& a, int mode, cudaStream_t s) {
 // Registers block size BW x BH of this translation unit in the size table.
 #define FFT3D_REGISTER_SIZE(BW, BH)                                                                     \
   static const bool fft3d_reg_##BW##x##BH = register_size(                                             \
-      SizeEntry{BW, BH, &fwd_sized<BW, BH>, &inv_sized<BW, BH>, &fused_sized<BW, BH>, &upload_twiddle_table, \
+      SizeEntry{BW, BH, &fwd_sized<BW, BH>, &inv_sized<BW, BH>, &frame_sized<BW, BH>, &upload_twiddle_table, \
                 &fwd_batch<BW, BH>, &inv_batch<BW, BH>, &ctas_per_plane<BW, BH>, &occupancy_of<BW, BH>,      \
                 &inv_frames<BW, BH>, &fwd_frames<BW, BH>, &inv_group<BW, BH>, &inv_group_batch<BW, BH>});
 
