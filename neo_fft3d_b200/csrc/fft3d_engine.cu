@@ -821,8 +821,12 @@ int pshow_frame(fft3d_plane* P, int n, const void* const src[5], const int strid
   return output_frame(P, P->d_tdom, tab, base, dst, dst_stride, cur, stride[2], host, false, st);
 }
 
-// Most blocks of a plane whose frames go in one launch (k_frame).
-constexpr int kOneLaunchBlocks = 600;
+// Most blocks of a plane whose frames go in one launch (k_frame): about three
+// CTAs per SM, one block each. One-frame calls, us per frame with one launch /
+// three, one plane and three planes on three streams: 48 x 48 blocks, 108
+// blocks 24 / 25 and 29 / 40, 374 blocks 27 / 27 and 40 / 40; 32 x 32 at bt = 5,
+// 336 blocks 19 / 23 and 25 / 40, 744 blocks 31 / 27 and 67 / 40.
+constexpr int kOneLaunchBlocks = 450;
 
 int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride[5], void* dst, int dst_stride,
                bool host, cudaStream_t st) {
@@ -953,7 +957,7 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
         fa.of.dst[0] = fs.dst[0] = fa.of.o.dst;
         fa.of.dst_stride[0] = fs.dst_stride[0] = dst_stride;
         fa.of.bytes = P->bytes;
-        fa.of.px4 = fft3d::overlap_add_frames_supported(fa.of.o, fs, P->bytes) ? 1 : 0;
+        fa.of.px = fft3d::overlap_add_pixels(fa.of.o, fs, P->bytes);
         fa.of.o.dst = nullptr;
         ola_done = true;
       }
@@ -1140,7 +1144,7 @@ bool fuse_run_ola(fft3d_plane* P, const fft3d::Deferred& d, const fft3d::Tempora
     ola_done[idx[k]] = 1;
   }
   of->bytes = d.ola[idx[0]].bytes;
-  of->px4 = fft3d::overlap_add_frames_supported(of->o, fs, of->bytes) ? 1 : 0;
+  of->px = fft3d::overlap_add_pixels(of->o, fs, of->bytes);
   return true;
 }
 

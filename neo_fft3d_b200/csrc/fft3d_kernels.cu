@@ -42,91 +42,19 @@ constexpr int kOla4BatchRows = 4 * kOlaTy;  // rows of one batched 4-pixel overl
 // fs (one frame per call, or a frame group's frames in one launch). V > 1
 // where the V pixels share their blocks and overlap case and their samples go
 // out in one store (overlap_add_width); the block column, its overlap case and
-// the synthesis windows along x are found once for the R rows. Each pixel's
-// arithmetic is overlap_add_px's, term for term, with the fused multiply-adds
-// that the compiler makes of it written out: three widths must round alike.
+// the synthesis windows along x are found once for the R rows (ola_pixels).
 // The planes whose block step is not a multiple of 4 (the filter's default
 // overlap of 10 with 32 x 32 blocks) had one launch per frame and one pixel per
 // thread: 344 us for 16 frames of 720p 16-bit 4:2:0, against 112 us here.
 template <typename T, int V, int R>
 __global__ void __launch_bounds__(kOlaTx * kOlaTy) k_overlap_add_rows(OlaArgs a, const __grid_constant__ OlaFrameSet fs) {
-  const Geom& g = a.g;
-  const int x0 = V * (blockIdx.x * kOlaTx + threadIdx.x);
-  if (x0 >= g.W) return;
-  const int X = g.sx + x0, bx = div_small(X, g.sx), x = X - bx * g.sx;
-  const bool xov = x < g.ow;
-  float sxr[V], sxl[V];
-#pragma unroll
-  for (int i = 0; i < V; i++) {
-    sxr[i] = xov ? __ldg(a.t.wsyn_xr + x + i) : 0.f;
-    sxl[i] = xov ? __ldg(a.t.wsyn_xl + x + i) : 0.f;
-  }
-  const int j = blockIdx.z;
-  const float* tdom = fs.tdom[j];
-  char* dst = static_cast<char*>(fs.dst[j]);
-  const long long stride = fs.dst_stride[j];
-  const int bw = g.bw, bh = g.bh;
-  const float norm = a.norm;
+  const int x0 = V * (blockIdx.x * kOlaTx + threadIdx.x), j = blockIdx.z;
+  if (x0 >= a.g.W) return;
+  const OlaColumn<V> c(a, x0);
 #pragma unroll
   for (int r = 0; r < R; r++) {
     const int k = (blockIdx.y * R + r) * kOlaTy + threadIdx.y;
-    if (k >= g.H) return;
-    const int Y = g.sy + k, by = div_small(Y, g.sy), y = Y - by * g.sy;
-    const bool yov = y < g.oh;
-    auto at = [&](int bxx, int byy, int yy, int xx, float (&v)[V]) {
-      if (!FFT3D_IN(bxx >= 0 && bxx < g.nox && byy >= 0 && byy < g.noy && yy >= 0 && yy < bh && xx >= 0 && xx + V <= bw,
-                    a.err)) {
-#pragma unroll
-        for (int i = 0; i < V; i++) v[i] = 0.f;
-        return;
-      }
-      const float* p = tdom + ((size_t)(byy * g.nox + bxx) * bh + yy) * bw + xx;
-      if constexpr (V == 4) {
-        const float4 q = ld_tdom4<false>(p);
-        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-      } else if constexpr (V == 2) {
-        asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(p));
-      } else {
-        v[0] = ld_tdom<false>(p);
-      }
-    };
-    float v[V], aa[V], b[V], c[V], d[V];
-    at(bx, by, y, x, d);
-    if (xov) at(bx - 1, by, y, x + g.sx, c);
-    if (!yov) {
-#pragma unroll
-      for (int i = 0; i < V; i++) {
-        const float t = xov ? fmaf(c[i], sxr[i], __fmul_rn(d[i], sxl[i])) : d[i];
-        v[i] = fmaf(t, norm, a.rounder) + a.base;
-      }
-    } else {
-      at(bx, by - 1, y + g.sy, x, b);
-      if (xov) at(bx - 1, by - 1, y + g.sy, x + g.sx, aa);
-      const float wr = __fmul_rn(__ldg(a.t.wsyn_yr + y), norm), wl = __fmul_rn(__ldg(a.t.wsyn_yl + y), norm);
-#pragma unroll
-      for (int i = 0; i < V; i++) {
-        const float u = xov ? fmaf(aa[i], sxr[i], __fmul_rn(b[i], sxl[i])) : b[i];
-        const float t = xov ? fmaf(c[i], sxr[i], __fmul_rn(d[i], sxl[i])) : d[i];
-        v[i] = fmaf(u, wr, __fmul_rn(t, wl)) + a.rounder + a.base;
-      }
-    }
-    const int fr = field_row(k, g.H, g.interlaced);
-    if (!FFT3D_IN(fr >= 0 && fr < g.H && x0 + V <= g.W, a.err)) return;
-    T o[V];
-#pragma unroll
-    for (int i = 0; i < V; i++) o[i] = clamp_sample<T>(v[i], a.maxval);
-    T* at_px = reinterpret_cast<T*>(dst + (long long)fr * stride) + x0;
-    if constexpr (V == 4) {
-      typename Pack4<T>::V q;
-      q.x = o[0], q.y = o[1], q.z = o[2], q.w = o[3];
-      *reinterpret_cast<typename Pack4<T>::V*>(at_px) = q;
-    } else if constexpr (V == 2) {
-      if constexpr (sizeof(T) == 1) *reinterpret_cast<uchar2*>(at_px) = make_uchar2(o[0], o[1]);
-      else if constexpr (sizeof(T) == 2) *reinterpret_cast<ushort2*>(at_px) = make_ushort2(o[0], o[1]);
-      else *reinterpret_cast<float2*>(at_px) = make_float2(o[0], o[1]);
-    } else {
-      *at_px = o[0];
-    }
+    if (k < a.g.H) ola_pixels<T, V, false>(a, c, fs.tdom[j], fs.dst[j], fs.dst_stride[j], x0, k);
   }
 }
 
@@ -171,7 +99,8 @@ __global__ void __launch_bounds__(kOlaTx * kOlaTy) k_overlap_add_batch(const Ola
     const OlaArgs a = args[it.x];  // private copy: fields stay in registers
     const int tx = (a.g.W + kOlaTx - 1) / kOlaTx;
     const int ty = it.y / tx, t = it.y - ty * tx;
-    overlap_add_px<T>(a, t * kOlaTx + threadIdx.x, ty * kOlaTy + threadIdx.y);
+    const int x0 = t * kOlaTx + threadIdx.x, k = ty * kOlaTy + threadIdx.y;
+    if (x0 < a.g.W && k < a.g.H) ola_pixels<T, 1, false>(a, OlaColumn<1>(a, x0), a.tdom, a.dst, a.dst_stride, x0, k);
   }
 }
 
@@ -186,11 +115,16 @@ __global__ void __launch_bounds__(kOlaTx * kOlaTy) k_overlap_add4_batch(const Ol
     const OlaArgs a = args[it.x];  // private copy: fields stay in registers
     const int tx = (a.g.W + 4 * kOlaTx - 1) / (4 * kOlaTx);
     const int ty = it.y / tx, t = it.y - ty * tx;
-    // kOla4BatchRows rows per item, so that the argument loads are shared by
-    // several pixel quads per thread
+    // kOla4BatchRows rows per item, so that the argument loads and the column
+    // are shared by several pixel quads per thread
+    const int x0 = 4 * (t * kOlaTx + threadIdx.x);
+    if (x0 >= a.g.W) continue;
+    const OlaColumn<4> c(a, x0);
 #pragma unroll
-    for (int r = 0; r < kOla4BatchRows; r += kOlaTy)
-      overlap_add_px4<T>(a, 4 * (t * kOlaTx + threadIdx.x), ty * kOla4BatchRows + r + threadIdx.y);
+    for (int r = 0; r < kOla4BatchRows; r += kOlaTy) {
+      const int k = ty * kOla4BatchRows + r + threadIdx.y;
+      if (k < a.g.H) ola_pixels<T, 4, false>(a, c, a.tdom, a.dst, a.dst_stride, x0, k);
+    }
   }
 }
 
@@ -404,14 +338,7 @@ int batch_occupancy(int bw, int bh, int which, int mode_or_bytes) {
   return e ? e->occupancy(which, mode_or_bytes) : 1;
 }
 
-bool overlap_add_frames_supported(const OlaArgs& a, const OlaFrameSet& fs, int bytes) {
-  if (fs.count < 1 || fs.count > kMaxGroupFrames) return false;
-  bool four = a.g.sx % 4 == 0 && a.g.ow % 4 == 0 && a.g.W % 4 == 0 && a.g.bw % 4 == 0;
-  for (int j = 0; j < fs.count && four; j++)
-    four = reinterpret_cast<uintptr_t>(fs.tdom[j]) % 16 == 0 &&
-           reinterpret_cast<uintptr_t>(fs.dst[j]) % (4 * bytes) == 0 && fs.dst_stride[j] % (4 * bytes) == 0;
-  return four;
-}
+int overlap_add_pixels(const OlaArgs& a, const OlaFrameSet& fs, int bytes) { return overlap_add_width(a, fs, bytes); }
 
 __global__ void k_fill(float* p, float v, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;

@@ -216,7 +216,7 @@ struct OlaFuse {
   unsigned epoch;                 // this launch's epoch (> 0)
   int tiles_x, tiles_y;
   int bytes;                      // sample size: 1, 2 or 4
-  int px4;                        // 4-pixel form (the plane meets its rules)
+  int px;                         // pixels per thread: 4, 2 or 1 (overlap_add_pixels)
 };
 
 // One output frame in one launch (k_frame). f.src/f.spec: the window's newest
@@ -280,8 +280,9 @@ cudaError_t launch_fill(float* p, float v, size_t n, cudaStream_t s);
 cudaError_t launch_overlap_add_frames(const OlaArgs& a, const OlaFrameSet& fs, int bytes_per_sample, cudaStream_t s);
 // Crop borders of a call's frames in one launch.
 cudaError_t launch_copy_borders(const BorderSet& bs, cudaStream_t s);
-// Whether every frame of fs meets the 4-pixel form's geometry and alignment rules.
-bool overlap_add_frames_supported(const OlaArgs& a, const OlaFrameSet& fs, int bytes_per_sample);
+// Adjacent pixels (4, 2 or 1) that share their blocks, their overlap case and
+// one aligned store in every frame of fs.
+int overlap_add_pixels(const OlaArgs& a, const OlaFrameSet& fs, int bytes_per_sample);
 // Batched forms (work items as in BatchLaunch); OLA items are 32x8-pixel tiles.
 cudaError_t launch_forward_batch(int bw, int bh, const BatchLaunch& l, int bytes_per_sample, cudaStream_t s);
 cudaError_t launch_filter_inverse_batch(int bw, int bh, const BatchLaunch& l, int mode, cudaStream_t s);

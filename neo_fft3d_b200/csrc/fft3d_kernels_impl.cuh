@@ -1202,75 +1202,7 @@ __device__ __forceinline__ float4 ld_tdom4(const float* p) {
   }
 }
 
-template <typename T>
-__device__ __forceinline__ void store_sample(T* p, float v, int maxval);
-template <>
-__device__ __forceinline__ void store_sample<uint8_t>(uint8_t* p, float v, int maxval) {
-  int i = __float2int_rz(v);  // C cast: truncation toward zero (src/buffer.cpp:406)
-  i = i < 0 ? 0 : (i > maxval ? maxval : i);
-  *p = (uint8_t)i;
-}
-template <>
-__device__ __forceinline__ void store_sample<uint16_t>(uint16_t* p, float v, int maxval) {
-  int i = __float2int_rz(v);
-  i = i < 0 ? 0 : (i > maxval ? maxval : i);
-  *p = (uint16_t)i;
-}
-template <>
-__device__ __forceinline__ void store_sample<float>(float* p, float v, int) {
-  float c = v < 0.f ? 0.f : v;  // float samples clamp to [0, 1] (src/buffer.cpp:397)
-  *p = c > 1.f ? 1.f : c;
-}
-
-// One thread per output pixel of the processed region: the (at most four)
-// blocks covering it, weighted with the synthesis windows and the FFT
-// normalisation in the association order of src/buffer.cpp:399-559.
-template <typename T, bool L2 = false>
-__device__ __forceinline__ void overlap_add_px(const OlaArgs& a, int x0, int k) {
-  const Geom& g = a.g;
-  if (x0 >= g.W || k >= g.H) return;
-  const int Y = g.sy + k, X = g.sx + x0;
-  const int by = div_small(Y, g.sy), y = Y - by * g.sy;
-  const int bx = div_small(X, g.sx), x = X - bx * g.sx;
-  const bool yov = y < g.oh, xov = x < g.ow;
-  const int bw = g.bw, bh = g.bh;
-  auto at = [&](int bxx, int byy, int yy, int xx) {
-    if (!FFT3D_IN(bxx >= 0 && bxx < g.nox && byy >= 0 && byy < g.noy && yy >= 0 && yy < bh && xx >= 0 && xx < bw,
-                  a.err))
-      return 0.f;
-    return ld_tdom<L2>(a.tdom + ((size_t)(byy * g.nox + bxx) * bh + yy) * bw + xx);
-  };
-  const float norm = a.norm;
-  float v;
-  if (!yov) {
-    const float d = at(bx, by, y, x);
-    if (!xov) v = d * norm + a.rounder + a.base;
-    else {
-      const float c = at(bx - 1, by, y, x + g.sx);
-      v = (c * __ldg(a.t.wsyn_xr + x) + d * __ldg(a.t.wsyn_xl + x)) * norm + a.rounder + a.base;
-    }
-  } else {
-    const float wr = __ldg(a.t.wsyn_yr + y) * norm, wl = __ldg(a.t.wsyn_yl + y) * norm;
-    const float b = at(bx, by - 1, y + g.sy, x), d = at(bx, by, y, x);
-    if (!xov) v = (b * wr + d * wl) + a.rounder + a.base;
-    else {
-      const float aa = at(bx - 1, by - 1, y + g.sy, x + g.sx), c = at(bx - 1, by, y, x + g.sx);
-      const float sxr = __ldg(a.t.wsyn_xr + x), sxl = __ldg(a.t.wsyn_xl + x);
-      v = ((aa * sxr + b * sxl) * wr + (c * sxr + d * sxl) * wl) + a.rounder + a.base;
-    }
-  }
-  const int fr = field_row(k, g.H, g.interlaced);
-  if (!FFT3D_IN(fr >= 0 && fr < g.H, a.err)) return;
-  T* row = reinterpret_cast<T*>(static_cast<char*>(a.dst) + (long long)fr * a.dst_stride);
-  store_sample<T>(row + x0, v, a.maxval);
-}
-
-// Four adjacent output pixels per thread (x0 a multiple of 4), for planes
-// whose block step, overlap, width and block width are multiples of 4 and
-// whose destination rows are aligned for a 4-sample store: the four pixels
-// share their blocks and overlap case, so the tdom reads are float4 loads,
-// the block indices are computed once and the samples go out in one store.
-// Each pixel's arithmetic is overlap_add_px's, term for term.
+// Four samples, as one store.
 template <typename T>
 struct Pack4;
 template <>
@@ -1298,94 +1230,98 @@ __device__ __forceinline__ T clamp_sample(float v, int maxval) {
   }
 }
 
-// The 4-pixel overlap-add in two steps, so that a thread can issue the block
-// reads of several pixel quads before it computes any of them: ola4_fetch
-// reads the (at most four) time-domain float4s of quad (x0, k) from `tdom`,
-// ola4_finish weights, sums, rounds and stores them.
-struct Ola4Px {
-  float4 aa, b, c, d;  // blocks (bx-1, by-1), (bx, by-1), (bx-1, by), (bx, by); zero where not read
-  int x, y;            // position inside the block step
-  bool xov, yov, ok;
-};
-
-template <bool L2>
-__device__ __forceinline__ Ola4Px ola4_fetch(const OlaArgs& a, const float* tdom, int x0, int k) {
-  const Geom& g = a.g;
-  Ola4Px p;
-  p.aa = p.b = p.c = p.d = make_float4(0.f, 0.f, 0.f, 0.f);
-  p.ok = x0 < g.W && k < g.H;
-  if (!p.ok) return p;
-  const int Y = g.sy + k, X = g.sx + x0;
-  const int by = div_small(Y, g.sy), bx = div_small(X, g.sx);
-  p.y = Y - by * g.sy;
-  p.x = X - bx * g.sx;
-  p.yov = p.y < g.oh;
-  p.xov = p.x < g.ow;
-  const int bw = g.bw, bh = g.bh;
-  auto at4 = [&](int bxx, int byy, int yy, int xx) {
-    if (!FFT3D_IN(bxx >= 0 && bxx < g.nox && byy >= 0 && byy < g.noy && yy >= 0 && yy < bh && xx >= 0 &&
-                      xx + 3 < bw,
-                  a.err))
-      return make_float4(0.f, 0.f, 0.f, 0.f);
-    return ld_tdom4<L2>(tdom + ((size_t)(byy * g.nox + bxx) * bh + yy) * bw + xx);
-  };
-  p.d = at4(bx, by, p.y, p.x);
-  if (p.xov) p.c = at4(bx - 1, by, p.y, p.x + g.sx);
-  if (p.yov) {
-    p.b = at4(bx, by - 1, p.y + g.sy, p.x);
-    if (p.xov) p.aa = at4(bx - 1, by - 1, p.y + g.sy, p.x + g.sx);
+// V adjacent pixels (V = 1, 2 or 4) of the processed region from column x0 on
+// that share their blocks and overlap case and go out in one store: what they
+// share along x ...
+template <int V>
+struct OlaColumn {
+  int bx, x;  // block column, position inside the block step
+  bool xov;
+  float sxr[V], sxl[V];  // synthesis windows
+  __device__ __forceinline__ OlaColumn(const OlaArgs& a, int x0) {
+    const int X = a.g.sx + x0;
+    bx = div_small(X, a.g.sx);
+    x = X - bx * a.g.sx;
+    xov = x < a.g.ow;
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+      sxr[i] = xov ? __ldg(a.t.wsyn_xr + x + i) : 0.f;
+      sxl[i] = xov ? __ldg(a.t.wsyn_xl + x + i) : 0.f;
+    }
   }
-  return p;
-}
-
-template <typename T>
-__device__ __forceinline__ void ola4_finish(const OlaArgs& a, void* dst, long long dst_stride, int x0, int k,
-                                            const Ola4Px& p) {
-  if (!p.ok) return;
+};
+// ... and those pixels of row k: the (at most four) blocks covering them,
+// weighted with the synthesis windows and the FFT normalisation in the
+// association order of src/buffer.cpp:399-559, with its fused multiply-adds
+// written out, so that every width rounds alike. Truncation toward zero, then
+// the clamp (src/buffer.cpp:397-406).
+template <typename T, int V, bool L2>
+__device__ __forceinline__ void ola_pixels(const OlaArgs& a, const OlaColumn<V>& q, const float* tdom, void* dst,
+                                           long long stride, int x0, int k) {
   const Geom& g = a.g;
-  const int x = p.x, y = p.y;
-  auto comp = [](const float4& q, int i) { return i == 0 ? q.x : (i == 1 ? q.y : (i == 2 ? q.z : q.w)); };
+  const int bw = g.bw, bh = g.bh, bx = q.bx, x = q.x;
   const float norm = a.norm;
-  float v[4];
-  if (!p.yov) {
-    if (!p.xov) {
+  const int Y = g.sy + k, by = div_small(Y, g.sy), y = Y - by * g.sy;
+  const bool yov = y < g.oh;
+  auto at = [&](int bxx, int byy, int yy, int xx, float (&v)[V]) {
+    if (!FFT3D_IN(bxx >= 0 && bxx < g.nox && byy >= 0 && byy < g.noy && yy >= 0 && yy < bh && xx >= 0 && xx + V <= bw,
+                  a.err)) {
 #pragma unroll
-      for (int i = 0; i < 4; i++) v[i] = comp(p.d, i) * norm + a.rounder + a.base;
+      for (int i = 0; i < V; i++) v[i] = 0.f;
+      return;
+    }
+    const float* p = tdom + ((size_t)(byy * g.nox + bxx) * bh + yy) * bw + xx;
+    if constexpr (V == 4) {
+      const float4 u = ld_tdom4<L2>(p);
+      v[0] = u.x, v[1] = u.y, v[2] = u.z, v[3] = u.w;
+    } else if constexpr (V == 2) {
+      if constexpr (L2) {
+        const float2 u = __ldcg(reinterpret_cast<const float2*>(p));
+        v[0] = u.x, v[1] = u.y;
+      } else {
+        asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(p));
+      }
     } else {
+      v[0] = ld_tdom<L2>(p);
+    }
+  };
+  float v[V], aa[V], b[V], c[V], d[V];
+  at(bx, by, y, x, d);
+  if (q.xov) at(bx - 1, by, y, x + g.sx, c);
+  if (!yov) {
 #pragma unroll
-      for (int i = 0; i < 4; i++)
-        v[i] = (comp(p.c, i) * __ldg(a.t.wsyn_xr + x + i) + comp(p.d, i) * __ldg(a.t.wsyn_xl + x + i)) * norm +
-               a.rounder + a.base;
+    for (int i = 0; i < V; i++) {
+      const float t = q.xov ? fmaf(c[i], q.sxr[i], __fmul_rn(d[i], q.sxl[i])) : d[i];
+      v[i] = fmaf(t, norm, a.rounder) + a.base;
     }
   } else {
-    const float wr = __ldg(a.t.wsyn_yr + y) * norm, wl = __ldg(a.t.wsyn_yl + y) * norm;
-    if (!p.xov) {
+    at(bx, by - 1, y + g.sy, x, b);
+    if (q.xov) at(bx - 1, by - 1, y + g.sy, x + g.sx, aa);
+    const float wr = __fmul_rn(__ldg(a.t.wsyn_yr + y), norm), wl = __fmul_rn(__ldg(a.t.wsyn_yl + y), norm);
 #pragma unroll
-      for (int i = 0; i < 4; i++) v[i] = (comp(p.b, i) * wr + comp(p.d, i) * wl) + a.rounder + a.base;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const float sxr = __ldg(a.t.wsyn_xr + x + i), sxl = __ldg(a.t.wsyn_xl + x + i);
-        v[i] = ((comp(p.aa, i) * sxr + comp(p.b, i) * sxl) * wr + (comp(p.c, i) * sxr + comp(p.d, i) * sxl) * wl) +
-               a.rounder + a.base;
-      }
+    for (int i = 0; i < V; i++) {
+      const float u = q.xov ? fmaf(aa[i], q.sxr[i], __fmul_rn(b[i], q.sxl[i])) : b[i];
+      const float t = q.xov ? fmaf(c[i], q.sxr[i], __fmul_rn(d[i], q.sxl[i])) : d[i];
+      v[i] = fmaf(u, wr, __fmul_rn(t, wl)) + a.rounder + a.base;
     }
   }
   const int fr = field_row(k, g.H, g.interlaced);
-  if (!FFT3D_IN(fr >= 0 && fr < g.H && x0 + 3 < g.W, a.err)) return;
-  T* row = reinterpret_cast<T*>(static_cast<char*>(dst) + (long long)fr * dst_stride);
-  typename Pack4<T>::V o;
-  o.x = clamp_sample<T>(v[0], a.maxval);
-  o.y = clamp_sample<T>(v[1], a.maxval);
-  o.z = clamp_sample<T>(v[2], a.maxval);
-  o.w = clamp_sample<T>(v[3], a.maxval);
-  *reinterpret_cast<typename Pack4<T>::V*>(row + x0) = o;
-}
-
-template <typename T, bool L2 = false>
-__device__ __forceinline__ void overlap_add_px4(const OlaArgs& a, int x0, int k) {
-  const Ola4Px p = ola4_fetch<L2>(a, a.tdom, x0, k);
-  ola4_finish<T>(a, a.dst, a.dst_stride, x0, k, p);
+  if (!FFT3D_IN(fr >= 0 && fr < g.H && x0 + V <= g.W, a.err)) return;
+  T o[V];
+#pragma unroll
+  for (int i = 0; i < V; i++) o[i] = clamp_sample<T>(v[i], a.maxval);
+  T* px = reinterpret_cast<T*>(static_cast<char*>(dst) + (long long)fr * stride) + x0;
+  if constexpr (V == 4) {
+    typename Pack4<T>::V w;
+    w.x = o[0], w.y = o[1], w.z = o[2], w.w = o[3];
+    *reinterpret_cast<typename Pack4<T>::V*>(px) = w;
+  } else if constexpr (V == 2) {
+    if constexpr (sizeof(T) == 1) *reinterpret_cast<uchar2*>(px) = make_uchar2(o[0], o[1]);
+    else if constexpr (sizeof(T) == 2) *reinterpret_cast<ushort2*>(px) = make_ushort2(o[0], o[1]);
+    else *reinterpret_cast<float2*>(px) = make_float2(o[0], o[1]);
+  } else {
+    *px = o[0];
+  }
 }
 
 // ---------------------------------------------------------------- bulk copies
@@ -1514,44 +1450,25 @@ __device__ __forceinline__ void group_filter_pair(const InverseArgs& a, size_t o
   }
 }
 
-// The overlap-add of output tile (tx, ty) (OlaFuse) for the run's frames:
-// overlap_add_px4 / overlap_add_px per pixel, the blocks read from L2.
-template <typename T>
-__device__ __noinline__ void group_ola_tile(const OlaFuse& of, const TemporalSet& ts, int count, int tx, int ty) {
+// The overlap-add of output tile (tx, ty) (OlaFuse) for the run's frames, V
+// pixels per thread, the blocks read from L2.
+template <typename T, int V>
+__device__ __forceinline__ void group_ola_tile_v(const OlaFuse& of, const TemporalSet& ts, int count, int tx, int ty) {
   const Geom& g = of.o.g;
   const int x_lo = (tx - 1) * g.sx, y_lo = (ty - 1) * g.sy;
-  const int wd = min(g.sx, g.W - x_lo), ht = min(g.sy, g.H - y_lo);
-  if (of.px4) {
-    // quads (frame j, row yy, quad xx); each thread fetches K of them before
-    // it finishes any, so that their L2 reads overlap
-    constexpr int K = 2;
-    const int q = (wd + 3) / 4, per = q * ht, total = count * per;
-    for (int i0 = threadIdx.x; i0 < total; i0 += K * blockDim.x) {
-      Ola4Px p[K];
-      int jj[K], xs[K], ks[K];
-#pragma unroll
-      for (int u = 0; u < K; u++) {
-        const int i = i0 + u * blockDim.x;
-        const int j = i < total ? i / per : 0, r = i - j * per, yy = r / q, xx = r - yy * q;
-        jj[u] = j;
-        xs[u] = i < total ? x_lo + 4 * xx : g.W;  // out of range: fetch and finish skip it
-        ks[u] = y_lo + yy;
-        p[u] = ola4_fetch<true>(of.o, ts.tdom[j], xs[u], ks[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < K; u++) ola4_finish<T>(of.o, of.dst[jj[u]], of.dst_stride[jj[u]], xs[u], ks[u], p[u]);
-    }
-    return;
-  }
+  const int wd = min(g.sx, g.W - x_lo) / V, ht = min(g.sy, g.H - y_lo);
+  // (V divides the step and the width: wd is exact)
   const int per = wd * ht;
   for (int i = threadIdx.x; i < count * per; i += blockDim.x) {
-    const int j = i / per, r = i - j * per, yy = r / wd, xx = r - yy * wd;
-    OlaArgs b = of.o;
-    b.tdom = ts.tdom[j];
-    b.dst = of.dst[j];
-    b.dst_stride = of.dst_stride[j];
-    overlap_add_px<T, true>(b, x_lo + xx, y_lo + yy);
+    const int j = i / per, r = i - j * per, yy = r / wd, x0 = x_lo + V * (r - yy * wd);
+    ola_pixels<T, V, true>(of.o, OlaColumn<V>(of.o, x0), ts.tdom[j], of.dst[j], of.dst_stride[j], x0, y_lo + yy);
   }
+}
+template <typename T>
+__device__ __noinline__ void group_ola_tile(const OlaFuse& of, const TemporalSet& ts, int count, int tx, int ty) {
+  if (of.px == 4) group_ola_tile_v<T, 4>(of, ts, count, tx, ty);
+  else if (of.px == 2) group_ola_tile_v<T, 2>(of, ts, count, tx, ty);
+  else group_ola_tile_v<T, 1>(of, ts, count, tx, ty);
 }
 
 // A thread's walk over the bin pairs of consecutive blocks, `STEP` pairs at a
@@ -1973,7 +1890,7 @@ __global__ void __launch_bounds__(kBulkWarps * 32) k_filter_inverse_bulk(Inverse
 // launches and the latency of three kernels' chains rather than any
 // throughput.
 template <int BW, int BH, typename T, int MODE>
-__global__ void __launch_bounds__(kWarps * 32, 3)
+__global__ void __launch_bounds__(kWarps * 32, ctas_for(5, group_smem_bytes<BW, BH>(1)))
     k_frame(const __grid_constant__ ForwardArgs f, const __grid_constant__ InverseArgs a,
             const __grid_constant__ TemporalSet ts, const __grid_constant__ OlaFuse of) {
   extern __shared__ __align__(16) float2 smem2[];
