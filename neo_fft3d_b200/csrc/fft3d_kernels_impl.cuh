@@ -455,20 +455,20 @@ __device__ __forceinline__ void forward_blocks(const ForwardArgs& a, int cta, co
   }
 }
 
-// Registers of the forward kernels: two packed rows of 32 samples are 64
-// registers, of 48 samples 96.
-template <int BW, int BH>
-__host__ __device__ constexpr int fwd_ctas(int extra) {
-  return ctas_for((BW > 32 || BH > 32 ? 15 : 20) * 32 / fwd_threads<BW>(), fwd_blocks<BW>() * BH * (BW / 2 + 1) * 8 + extra);
-}
 template <int BW, int BH>
 __host__ __device__ constexpr int fwd_smem() { return fwd_blocks<BW>() * BH * (BW / 2 + 1) * 8; }
+// CTAs per SM: two packed rows of 32 samples are 64 registers (20 warps, 96
+// registers a thread), of 48 samples 96 (15 warps).
+template <int BW, int BH>
+__host__ __device__ constexpr int fwd_ctas() {
+  return ctas_for((BW > 32 || BH > 32 ? 15 : 20) * 32 / fwd_threads<BW>(), fwd_smem<BW, BH>());
+}
 
 // The new frames of one or more output frames in one launch: CTA x transforms
 // CTA x % fs.ctas of frame x / fs.ctas (one launch instead of one per frame,
 // so the grid has no per-frame wave tail).
 template <int BW, int BH, typename T>
-__global__ void __launch_bounds__(fwd_threads<BW>(), (fwd_ctas<BW, BH>(0)))
+__global__ void __launch_bounds__(fwd_threads<BW>(), (fwd_ctas<BW, BH>()))
     k_forward_frames(const __grid_constant__ ForwardArgs a, const __grid_constant__ FwdFrameSet fs) {
   const int j = blockIdx.x / fs.ctas, c = blockIdx.x - j * fs.ctas;
   forward_blocks<BW, BH, T>(a, c, FrameFwd{fs.src[j], fs.stride[j], fs.spec[j]});
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(fwd_threads<BW>(), (fwd_ctas<BW, BH>(0)))
 // Batched forward: work item i = (plane, CTA of that plane); the grid walks
 // the items (persistent when the grid is smaller than the item count).
 template <int BW, int BH, typename T>
-__global__ void __launch_bounds__(fwd_threads<BW>(), (fwd_ctas<BW, BH>((int)sizeof(ForwardArgs))))
+__global__ void __launch_bounds__(fwd_threads<BW>(), (ctas_for(16 * 32 / fwd_threads<BW>(), fwd_smem<BW, BH>() + (int)sizeof(ForwardArgs))))
     k_forward_batch(const ForwardArgs* __restrict__ args, const int2* __restrict__ items, int nitems) {
   // the item's arguments staged in shared memory: the body's stores cannot
   // alias them, and they cost no registers
@@ -818,11 +818,8 @@ __device__ __forceinline__ Pair filter_pair(const Pair (&w)[5], const Pair& grid
   }
 }
 
-// sharpen_bin of a pair; wsh, wdh: the pair's weights.
-__device__ __forceinline__ Pair sharpen_pair(const InverseArgs& a, const Pair& v, const Pair& grid, f2x wsh, f2x wdh,
-                                             float gf) {
-  const Pair gc = pscale_kept(grid, dup2(gf)), c = psub(v, gc);
-  const f2x psd = ppsd(c);
+// sharpen_fact x dehalo_fact (those that are on) of a pair of power spectra
+__device__ __forceinline__ f2x sharpen_factor(const InverseArgs& a, f2x psd, f2x wsh, f2x wdh) {
   f2x f = kc(kOne);
   if (a.c.use_sharpen) {
     const f2x smax = dup2(a.c.smax2n);
@@ -835,6 +832,25 @@ __device__ __forceinline__ Pair sharpen_pair(const InverseArgs& a, const Pair& v
     const f2x d = mul2(top, rcp2(fma2(mul2(dup2(a.c.dehalo), wdh), psd, top)));
     f = a.c.use_sharpen ? mul2(f, d) : d;
   }
+  return f;
+}
+
+// sharpen_bin of a pair; wsh, wdh: the pair's weights.
+__device__ __forceinline__ Pair sharpen_pair(const InverseArgs& a, const Pair& v, const Pair& grid, f2x wsh, f2x wdh,
+                                             float gf) {
+  const Pair gc = pscale_kept(grid, dup2(gf)), c = psub(v, gc);
+  const f2x f = sharpen_factor(a, ppsd(c), wsh, wdh);
+  return Pair{fma2(c.re, f, gc.re), fma2(c.im, f, gc.im)};
+}
+
+// filter_vals<MODE_WIENER2D> of a pair, the sharpen/dehalo factors in its
+// Wiener factor where the filter fuses them.
+__device__ __forceinline__ Pair wiener2d_pair(const InverseArgs& a, const Pair& v, const Pair& grid, float gf, f2x nn,
+                                              f2x wsh, f2x wdh) {
+  const Pair gc = pscale_kept(grid, dup2(gf)), c = psub(v, gc);
+  const f2x psd = ppsd(c);
+  f2x f = max2(fma2(nn, rcp2(psd), kc(kOne)), a.c.lowlimit);
+  if (a.c.fuse_sharpen && (a.c.use_sharpen || a.c.use_dehalo)) f = mul2(f, sharpen_factor(a, psd, wsh, wdh));
   return Pair{fma2(c.re, f, gc.re), fma2(c.im, f, gc.im)};
 }
 
@@ -872,15 +888,10 @@ __device__ __forceinline__ float4 group_filter_one(const InverseArgs& a, size_t 
     for (int k = 0; k < 5; k++) w[k] = pair_of(r[k >= LO && k <= HI ? k : LO]);
     return bins_of(filter_pair<MODE>(w, pair_grid(a, bin), gf, pair_noise<MODE>(a, off, bin), a.c.lowlimit));
   } else if constexpr (MODE == MODE_WIENER2D) {
-    float2 w0[5], w1[5];
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-      w0[k] = k == 2 ? make_float2(r[2].x, r[2].y) : make_float2(0.f, 0.f);
-      w1[k] = k == 2 ? make_float2(r[2].z, r[2].w) : make_float2(0.f, 0.f);
-    }
-    const float2 v0 = filter_vals<MODE>(a, w0, off, bin, gf, bin_tab<MODE>(a, bin), false);
-    const float2 v1 = filter_vals<MODE>(a, w1, off, bin + 1, gf, bin_tab<MODE>(a, bin + 1), false);
-    return make_float4(v0.x, v0.y, v1.x, v1.y);
+    const bool fuse = a.c.fuse_sharpen;
+    return bins_of(wiener2d_pair(a, pair_of(r[2]), pair_grid(a, bin), gf, pair_noise<MODE>(a, off, bin),
+                                 pair_weights(a.t.wsharpen, fuse && a.c.use_sharpen, bin),
+                                 pair_weights(a.t.wdehalo, fuse && a.c.use_dehalo, bin)));
   } else {
     return r[2];
   }
