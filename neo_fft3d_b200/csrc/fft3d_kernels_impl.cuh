@@ -15,17 +15,12 @@ namespace {
 
 constexpr int kWarps = 4;       // warps per CTA in k_forward / k_filter_inverse
 
-// CTAs per SM that the frame-group forward and filter/inverse kernels are
-// compiled for, where their shared memory lets that many reside (register
-// budget 65536 / (128 x CTAs): 80 registers at 6). Measured at 1080p bt=5
-// bw=32: 6 for both is 2.5 % faster than 5 (the filter/inverse spills 88
-// bytes but gains a sixth CTA).
-#ifndef FFT3D_GROUP_CTAS
-#define FFT3D_GROUP_CTAS 6
-#endif
-// ... and for short Wiener 3D runs, whose threads hold two windows (the one
-// they filter and the next one's loads in flight)
-constexpr int kShortCtas = 5;
+// CTAs per SM that the filter/inverse kernels are compiled for, where their
+// shared memory lets that many reside: walks of a Wiener 3D run (whose tiles
+// allow 4 at 32 x 32 and bt = 5), and the others at 96 registers (at 6 CTAs and
+// 80 registers they spill 52 bytes: 1080p bt=5 with its spatial edge frames
+// 1820 us per 24 frames, 1763 at 5).
+constexpr int kWalkCtas = 6, kShortCtas = 5;
 // shared memory per SM, and what the runtime reserves per resident CTA
 constexpr int kSmemPerSm = 228 * 1024, kSmemPerCtaReserved = 1024;
 __host__ __device__ constexpr int ctas_for(int want, int smem_per_cta) {
@@ -1513,7 +1508,7 @@ __host__ __device__ constexpr int run_tiles() {
 }
 template <int BW, int BH, int MODE, bool STAGED>
 __host__ __device__ constexpr int run_ctas(int extra) {
-  return ctas_for(STAGED || MODE < 2 ? FFT3D_GROUP_CTAS : kShortCtas,
+  return ctas_for(STAGED && MODE >= 2 ? kWalkCtas : kShortCtas,
                   group_smem_bytes<BW, BH>(run_tiles<BW, BH, MODE, STAGED>()) + extra);
 }
 
