@@ -102,13 +102,10 @@ int fft3d_plane_filter_device(fft3d_plane* h, int n, const void* const src[5], c
  * where the frame's spectrum is cached); frame n0 + j is written to dst[j]
  * (stride dst_stride[j]); all work is queued on `stream` (NULL = the
  * handle's own stream). On the default and tensor-core paths, the group's
- * new frames are transformed by one launch and its overlap-adds are one
- * launch; Wiener 3D
- * planes (bt = 2..5) filter the group's frames with one filter/inverse launch
- * whose CTAs interleave the frames block range by block range, so that a
- * window spectrum shared by up to bt frames is read from HBM about once
- * (Kalman, Wiener 2D and sharpen-only planes: one filter/inverse launch per
- * frame, in frame order). The ring keeps every spectrum the group needs and
+ * new frames are transformed by one launch, its overlap-adds are one launch,
+ * and each run of consecutive frames of one filter mode (Kalman in frame
+ * order) is one filter/inverse launch that reads each window spectrum from HBM
+ * about once for the run. The ring keeps every spectrum the group needs and
  * there is one time-domain buffer per frame (both grow on first use:
  * count + bt spectra and count - 1 buffers). Planes on the other paths
  * (fused, learned PSD, bulk-staged) filter the frames one after another.

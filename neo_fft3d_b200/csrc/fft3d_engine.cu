@@ -48,6 +48,13 @@ int cuda_fail(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail(e_, what); \
   } while (0)
 
+// Most blocks of a plane whose frames go in one launch (k_frame): about three
+// CTAs per SM, one block each. One-frame calls, us per frame with one launch /
+// three, one plane and three planes on three streams: 48 x 48 blocks, 108
+// blocks 24 / 25 and 29 / 40, 374 blocks 27 / 27 and 40 / 40; 32 x 32 at bt = 5,
+// 336 blocks 19 / 23 and 25 / 40, 744 blocks 31 / 27 and 67 / 40.
+constexpr int kOneLaunchBlocks = 450;
+
 struct Slot {
   float2* spec = nullptr;
   int frame = -1;
@@ -102,13 +109,12 @@ struct fft3d_plane {
   // launch for the run, then a sharpen/inverse launch; 0 (=fused): one
   // filter/inverse launch per Wiener 3D run, frames interleaved by CTA
   int group_split = 2;
-  // NEO_FFT3D_FUSED_OLA=1: a run's overlap-adds are done by its
-  // filter/inverse launch instead of a separate overlap-add launch (measured
-  // slower: the tile overlap-adds at the CTAs' tails are latency-bound);
-  // per-tile arrival counters (nox x noy, zeroed once) and the launch epoch
-  // their targets count in
+  // per-tile arrival counters (nox x noy, zero between launches) of
+  // overlap-adds done by the launch that makes their blocks: one-launch frames
+  // of small planes, and with NEO_FFT3D_FUSED_OLA=1 the frame groups' runs
+  // (measured slower on large planes: the tile overlap-adds at the CTAs' tails
+  // are latency-bound)
   unsigned* d_ola_cnt = nullptr;
-  unsigned ola_epoch = 0;
   bool fuse_ola = false;
   int occ = 0;
   int keep_lo = 1, keep_hi = 0;
@@ -185,12 +191,12 @@ struct fft3d_plane {
   std::vector<cudaEvent_t> sync_pool;
   uint64_t frames_done = 0;
   // kernel sequence of one output frame (NEO_FFT3D_PATH = unfused (default) | split | fused):
-  //   split:   k_forward (new frame), k_filter_bins (streaming filter of all
+  //   split:   the forward (new frame), k_filter_bins (streaming filter of all
   //            bins into d_filt), k_filter_inverse<sharpen only> on d_filt
-  //   unfused: k_forward, k_filter_inverse (filter + sharpen + inverse)
+  //   unfused: the forward, the filter/inverse (filter + sharpen + inverse)
   //   fused:   k_frame (new frame's forward + filter + inverse in one launch)
   //   tc:      as unfused, with the forward transform on the tensor cores
-  //            (k_forward_tc, 32x32 blocks; other sizes fall back to k_forward)
+  //            (k_forward_tc, 32x32 blocks; other sizes fall back to the FP32 one)
   int path = 1;  // 0 split, 1 unfused, 2 fused, 3 tc
   uint8_t* d_tc = nullptr;  // tensor-core DFT tables (path 3)
   int* d_err = nullptr;     // device error flag (tensor-core waits: bit 0, bulk-copy waits: bit 1)
@@ -611,37 +617,15 @@ fft3d::OlaArgs ola_args(const fft3d_plane* P, const float* tdom, const fft3d::Ta
 }
 
 // The arrival counters of overlap-adds done by the launch that makes their
-// blocks, and the launch's epoch: false when the plane's output tiles are not
-// inside its block grid or the counters cannot be had.
-bool next_ola_epoch(fft3d_plane* P, fft3d::OlaFuse* of, cudaStream_t st) {
+// blocks: false when the plane's output tiles are not inside its block grid or
+// it has no counters (they are allocated with the plane, so that a call
+// allocates nothing and can be captured).
+bool ola_fuse_setup(const fft3d_plane* P, fft3d::OlaFuse* of) {
   const fft3d::Geom& g = P->g;
   of->tiles_x = (g.sx + g.W - 1) / g.sx;
   of->tiles_y = (g.sy + g.H - 1) / g.sy;
-  if (of->tiles_x < 1 || of->tiles_y < 1 || of->tiles_x >= g.nox || of->tiles_y >= g.noy) return false;
-  const size_t cnt_bytes = (size_t)g.nblocks * sizeof(unsigned);
-  if (!P->d_ola_cnt) {
-    if (dmalloc(P, &P->d_ola_cnt, cnt_bytes) != cudaSuccess) {
-      cudaGetLastError();
-      P->d_ola_cnt = nullptr;
-      return false;
-    }
-    if (cudaMemsetAsync(P->d_ola_cnt, 0, cnt_bytes, st) != cudaSuccess) {
-      cudaGetLastError();
-      dfree(P, P->d_ola_cnt, cnt_bytes);
-      P->d_ola_cnt = nullptr;
-      return false;
-    }
-    P->ola_epoch = 0;
-  }
-  if (P->ola_epoch >= (1u << 29)) {  // targets stay below 2^32: start the counts over
-    if (cudaMemsetAsync(P->d_ola_cnt, 0, cnt_bytes, st) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    P->ola_epoch = 0;
-  }
+  if (!P->d_ola_cnt || of->tiles_x < 1 || of->tiles_y < 1 || of->tiles_x >= g.nox || of->tiles_y >= g.noy) return false;
   of->cnt = P->d_ola_cnt;
-  of->epoch = ++P->ola_epoch;
   return true;
 }
 
@@ -821,13 +805,6 @@ int pshow_frame(fft3d_plane* P, int n, const void* const src[5], const int strid
   return output_frame(P, P->d_tdom, tab, base, dst, dst_stride, cur, stride[2], host, false, st);
 }
 
-// Most blocks of a plane whose frames go in one launch (k_frame): about three
-// CTAs per SM, one block each. One-frame calls, us per frame with one launch /
-// three, one plane and three planes on three streams: 48 x 48 blocks, 108
-// blocks 24 / 25 and 29 / 40, 374 blocks 27 / 27 and 40 / 40; 32 x 32 at bt = 5,
-// 336 blocks 19 / 23 and 25 / 40, 744 blocks 31 / 27 and 67 / 40.
-constexpr int kOneLaunchBlocks = 450;
-
 int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride[5], void* dst, int dst_stride,
                bool host, cudaStream_t st) {
   if (P->reset_pending) {  // fft3d_plane_reset queued on the plane's stream
@@ -949,7 +926,7 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
       fa.f = forward_args(P, new_src, new_stride, news->spec);
       fa.v = ia;
       fa.of = fft3d::OlaFuse{};
-      if (small && next_ola_epoch(P, &fa.of, st)) {
+      if (small && ola_fuse_setup(P, &fa.of)) {
         fa.of.o = ola_args(P, nullptr, P->tab, fa.f.base, dst, dst_stride);
         fft3d::OlaFrameSet fs{};
         fs.count = 1;
@@ -964,9 +941,7 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
       {
         const double pix = (double)P->g.W * P->g.H * P->bytes;
         TimeScope ts(P, K_FUSED, pix + (to - from) * S + S + state + (ola_done ? pix : T), st);
-        const cudaError_t le = fft3d::launch_frame(fa, mode, P->bytes, st);
-        if (le != cudaSuccess && ola_done) P->ola_epoch--;  // no arrivals were counted for this epoch
-        CK(le, "one-launch kernel");
+        CK(fft3d::launch_frame(fa, mode, P->bytes, st), "one-launch kernel");
       }
       if (host) CK(cudaEventRecord(P->cur->in_free, st), "event");
     } else if (P->path == 0 && mode != fft3d::MODE_SHARPEN_ONLY) {
@@ -1129,7 +1104,7 @@ bool fuse_run_ola(fft3d_plane* P, const fft3d::Deferred& d, const fft3d::Tempora
     idx[k - i] = m;
   }
   *of = fft3d::OlaFuse{};
-  if (!next_ola_epoch(P, of, st)) return false;
+  if (!ola_fuse_setup(P, of)) return false;
   of->o = d.ola[idx[0]].a;
   of->o.tdom = nullptr;
   of->o.dst = nullptr;
@@ -1233,9 +1208,7 @@ int run_group(fft3d_plane* P, const fft3d::Deferred& d, cudaStream_t st) {
     TimeScope tsc(P, K_INVERSE, (double)seen.size() * S + state + n * (fused ? pix : T), st);
     fft3d::InverseArgs ga = d.inv[i].a;
     for (auto& p : ga.in) p = nullptr;
-    const cudaError_t le = fft3d::launch_filter_inverse_group(ga, ts, mode, st, fused ? &of : nullptr);
-    if (le != cudaSuccess && fused) P->ola_epoch--;  // no arrivals were counted for this epoch
-    CK(le, "filter/inverse kernel (frame group)");
+    CK(fft3d::launch_filter_inverse_group(ga, ts, mode, st, fused ? &of : nullptr), "filter/inverse kernel (frame group)");
     g_launches++;
     i = e;
   }
@@ -1868,6 +1841,22 @@ int fft3d_plane_create(const fft3d_params* p, const fft3d_plane_desc* d, int dev
     if (cudaEventCreateWithFlags(&sg.in_free, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&sg.out_free, cudaEventDisableTiming) != cudaSuccess)
       return bail(fail(FFT3D_E_CUDA, "neo_fft3d: event creation failed"));
+  }
+  // Arrival counters (ola_fuse_setup), a few KB: without them the overlap-adds
+  // are launches of their own, so a failure here is none, and the allocation
+  // cap does not count them.
+  if (P->fuse_ola || (P->path == 1 && g.nblocks <= kOneLaunchBlocks)) {
+    const size_t cnt_bytes = (size_t)g.nblocks * sizeof(unsigned);
+    // (zeroed on the plane's stream: the first call waits for the reset queued there below)
+    if (cudaMalloc(&P->d_ola_cnt, cnt_bytes) == cudaSuccess &&
+        cudaMemsetAsync(P->d_ola_cnt, 0, cnt_bytes, P->stream) == cudaSuccess) {
+      P->alloc_used += cnt_bytes;
+      if (P->alloc_cap) P->alloc_cap += cnt_bytes;
+    } else {
+      cudaGetLastError();
+      cudaFree(P->d_ola_cnt);
+      P->d_ola_cnt = nullptr;
+    }
   }
   *out = P;
   if ((rc = fft3d_plane_reset(P))) { *out = nullptr; return bail(rc); }

@@ -1,20 +1,25 @@
 // Device kernels of the FFT3D filtering core (sm_100a, FP32 CUDA-core path).
 //
-// Per plane and output frame the hot path is three kernels:
-//   k_forward         frame -> mirrored cover -> windowed overlapped blocks ->
-//                     2D r2c FFT -> one slot of the device spectrum ring
-//                     (replaces FrameToCover + CoverToOverlap + FFTW r2c,
-//                     src/buffer.cpp:6-379, src/fft3d_engine.h:616-618,661-664)
-//   k_filter_inverse  Wiener 2D / 3D2..3D5, Kalman or sharpen-only filter of
-//                     every bin, sharpen/dehalo, 2D c2r -> time-domain blocks
-//                     (replaces Apply*/Kalman/Sharpen C kernels and FFTW c2r,
-//                     src/code_impl/*.cpp, src/fft3d_engine.h:669-674)
-//   k_overlap_add     synthesis window, overlap-add, rounding and clamped
-//                     8/16-bit (or float) write-back of the plane interior
-//                     (replaces OverlapToCover + CoverToFrame, src/buffer.cpp:382-600)
+// The hot path of a plane is three launches, for one frame or for a group of
+// frames (one launch in all, k_frame, for one frame of a small plane):
+//   forward         frame -> mirrored cover -> windowed overlapped blocks ->
+//                   2D r2c FFT -> one slot of the device spectrum ring
+//                   (k_forward_frames, k_forward_batch; replaces FrameToCover +
+//                   CoverToOverlap + FFTW r2c, src/buffer.cpp:6-379,
+//                   src/fft3d_engine.h:616-618,661-664)
+//   filter/inverse  Wiener 2D / 3D2..3D5, Kalman or sharpen-only filter of
+//                   every bin, sharpen/dehalo, 2D c2r -> time-domain blocks
+//                   (k_filter_inverse_group, one CTA per block for a run of
+//                   frames; k_filter_inverse, one warp per block, for one frame
+//                   of a large plane; replaces Apply*/Kalman/Sharpen C kernels
+//                   and FFTW c2r, src/code_impl/*.cpp, src/fft3d_engine.h:669-674)
+//   overlap-add     synthesis window, overlap-add, rounding and clamped
+//                   8/16-bit (or float) write-back of the plane interior
+//                   (k_overlap_add_rows; replaces OverlapToCover + CoverToFrame,
+//                   src/buffer.cpp:382-600)
 //
-// One warp owns one block in the two FFT kernels; its tiles are staged in
-// shared memory so that every global access is coalesced.
+// The FFT kernels' tiles are staged in shared memory so that every global
+// access is coalesced.
 #pragma once
 #include <cstdint>
 #include <string>
@@ -139,7 +144,7 @@ struct FilterFrameSet {
 
 // A run of consecutive output frames n0 .. n0 + count - 1 (count <=
 // kGroupTile) of one plane with one mode, filtered and inverse-transformed
-// by one launch with one CTA per block (k_filter_inverse_group): spec[s] is
+// by one launch, each block's frames in one CTA (k_filter_inverse_group): spec[s] is
 // the spectrum of frame n0 - 2 + s (null where no window of the run reaches),
 // tdom[j] receives frame n0 + j's time-domain blocks.
 constexpr int kGroupTile = 8;
@@ -205,15 +210,14 @@ struct OlaArgs {
 // whose blocks are (tx, ty), (tx-1, ty) when ow > 0, (tx, ty-1) when oh > 0
 // and (tx-1, ty-1) when both. Each CTA adds one arrival to the counter of
 // every tile its block feeds once its time-domain blocks are stored; the CTA
-// that brings a counter to the tile's block count times the launch's epoch
-// (so the counters need no reset between launches) does that tile's
-// overlap-add for all the run's frames, from L2.
+// that brings a counter to the tile's block count sets it back to zero (for
+// the next launch) and does that tile's overlap-add for all the run's frames,
+// from L2.
 struct OlaFuse {
   OlaArgs o;                      // shared arguments (o.tdom, o.dst unused)
   void* dst[kGroupTile];          // frame j's destination plane at the crop origin
   long long dst_stride[kGroupTile];
-  unsigned* cnt;                  // arrival counters, indexed ty * nox + tx
-  unsigned epoch;                 // this launch's epoch (> 0)
+  unsigned* cnt;                  // arrival counters, indexed ty * nox + tx, zero between launches
   int tiles_x, tiles_y;
   int bytes;                      // sample size: 1, 2 or 4
   int px;                         // pixels per thread: 4, 2 or 1 (overlap_add_pixels)

@@ -13,7 +13,7 @@
 namespace fft3d {
 namespace {
 
-constexpr int kWarps = 4;       // warps per CTA in k_forward / k_filter_inverse
+constexpr int kWarps = 4;       // warps per CTA of the forward and filter/inverse kernels
 
 // CTAs per SM that the filter/inverse kernels are compiled for, where their
 // shared memory lets that many reside: walks of a Wiener 3D run (whose tiles
@@ -1733,8 +1733,11 @@ __device__ __forceinline__ bool filter_inverse_group_cta(const InverseArgs& a, c
       if ((dx == 0 || a.g.ow > 0) && (dy == 0 || a.g.oh > 0) && tx >= 1 && tx <= of->tiles_x && ty >= 1 &&
           ty <= of->tiles_y && FFT3D_IN(tx < a.g.nox && ty < a.g.noy, a.err)) {
         __threadfence();
-        last = atomicAdd(of->cnt + ty * a.g.nox + tx, 1u) + 1u == need * of->epoch;
-        if (last) __threadfence();
+        last = atomicAdd(of->cnt + ty * a.g.nox + tx, 1u) + 1u == need;
+        if (last) {
+          of->cnt[ty * a.g.nox + tx] = 0;  // ready for the next launch, a graph's replay too
+          __threadfence();
+        }
       }
       done[t] = last;
     }
@@ -2012,7 +2015,7 @@ cudaError_t fwd_sized(const ForwardArgs& a, int bytes, cudaStream_t s) {
 }
 
 inline bool ola_fuse_ok(const OlaFuse& of, const Geom& g) {
-  return of.cnt && of.epoch != 0 && of.tiles_x >= 1 && of.tiles_y >= 1 && of.tiles_x < g.nox && of.tiles_y < g.noy &&
+  return of.cnt && of.tiles_x >= 1 && of.tiles_y >= 1 && of.tiles_x < g.nox && of.tiles_y < g.noy &&
          (of.bytes == 1 || of.bytes == 2 || of.bytes == 4);
 }
 

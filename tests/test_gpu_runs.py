@@ -99,3 +99,50 @@ def test_overlap_add_widths_and_borders(gpu, w, bw, ow, crop, bits):
     assert (d <= 1).mean() >= 0.999 and d.max() <= 3, ((d <= 1).mean(), d.max())
     for sizes in ([13], [4]):
         assert np.array_equal(ref, _filter(torch, a, bits, filt, sizes)), sizes
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h", [(176, 144), (640, 480)])
+def test_captured_call_replays(gpu, w, h):
+    """A one-frame device call captured in a CUDA graph (small planes: one
+    launch with arrival counters; larger ones: three launches) gives the frame
+    of whatever its source holds at each replay."""
+    import torch
+    a = synth.make_clip(w, h, 4, noise_sigma=5.0, seed=9, planes=1)[0]
+    filt = dict(sigma=2.5, bt=1, bw=32, bh=32, ow=16, oh=16, sharpen=0.3)
+    want = [_filter_one(torch, a[k], filt) for k in range(4)]
+    e = engine.PlaneEngine(make_params(**filt), plane_descs([a.shape[1:]], 8, 4)[0])
+    src = torch.from_numpy(a[0]).cuda()
+    out = torch.empty_like(src)
+    s = torch.cuda.Stream()
+    call = lambda n: e.filter_device(n, [0, 0, src.data_ptr(), 0, 0], [w] * 5, out.data_ptr(), w, s.cuda_stream)  # noqa: E731
+    with torch.cuda.stream(s):
+        call(0)  # kernels loaded, the plane's reset passed
+        s.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            call(1)
+        for k in (1, 2, 3, 0, 0):
+            src.copy_(torch.from_numpy(a[k]))
+            out.fill_(1)
+            graph.replay()
+            s.synchronize()
+            assert np.array_equal(out.cpu().numpy(), want[k]), k
+        # a plain call afterwards (which also records the plane's last work outside the capture)
+        src.copy_(torch.from_numpy(a[2]))
+        call(2)
+        s.synchronize()
+        assert np.array_equal(out.cpu().numpy(), want[2])
+    del graph
+    e.close()
+
+
+def _filter_one(torch, frame, filt):
+    e = engine.PlaneEngine(make_params(**filt), plane_descs([frame.shape], 8, 1)[0])
+    src = torch.from_numpy(frame).cuda()
+    out = torch.full_like(src, 1)
+    w = frame.shape[1]
+    e.filter_device(0, [0, 0, src.data_ptr(), 0, 0], [w] * 5, out.data_ptr(), w)
+    e.synchronize()
+    e.close()
+    return out.cpu().numpy()
