@@ -90,7 +90,9 @@ int fft3d_plane_filter(fft3d_plane* h, int n, const void* const src[5], const in
  * a host synchronisation. A plane's calls are queued one at a time (its lock);
  * their GPU work is ordered when they use one stream, as the spectrum ring and
  * the Kalman state carry over from call to call: a caller that switches
- * streams orders them itself (an event). */
+ * streams orders them itself (an event).
+ * dst may be one of the call's source planes (a frame filtered in place): every
+ * pixel is read before any is written. */
 int fft3d_plane_filter_device(fft3d_plane* h, int n, const void* const src[5], const int src_stride[5], void* dst,
                               int dst_stride, void* stream);
 

@@ -629,6 +629,21 @@ bool ola_fuse_setup(const fft3d_plane* P, fft3d::OlaFuse* of) {
   return true;
 }
 
+// Whether two planes' rows share memory (by their address ranges: rows of one
+// that lie between the other's count too).
+bool planes_meet(const fft3d_plane* P, const void* a, long long astride, const void* b, long long bstride) {
+  const long long row = (long long)P->d.width * P->bytes;
+  auto range = [&](const void* p, long long stride, uintptr_t* lo, uintptr_t* hi) {
+    const long long last = (long long)(P->d.height - 1) * stride;
+    *lo = reinterpret_cast<uintptr_t>(p) + std::min(last, 0LL);
+    *hi = reinterpret_cast<uintptr_t>(p) + std::max(last, 0LL) + row;
+  };
+  uintptr_t a0, a1, b0, b1;
+  range(a, astride, &a0, &a1);
+  range(b, bstride, &b0, &b1);
+  return a0 < b1 && b0 < a1;
+}
+
 // The output of one frame from its time-domain blocks: the crop borders from
 // the source frame (src/fft3d.hpp:292-352), the overlap-add with the tables'
 // synthesis windows and sample offset `base`, and on the host path the
@@ -926,7 +941,11 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
       fa.f = forward_args(P, new_src, new_stride, news->spec);
       fa.v = ia;
       fa.of = fft3d::OlaFuse{};
-      if (small && ola_fuse_setup(P, &fa.of)) {
+      // (a frame filtered in place keeps its overlap-add as a launch of its
+      // own: the arrivals order a tile after the blocks that make it, not after
+      // the blocks that still read its pixels for their transforms, such as
+      // those mirrored at the plane's edges)
+      if (small && !planes_meet(P, dst, dst_stride, new_src, new_stride) && ola_fuse_setup(P, &fa.of)) {
         fa.of.o = ola_args(P, nullptr, P->tab, fa.f.base, dst, dst_stride);
         fft3d::OlaFrameSet fs{};
         fs.count = 1;
