@@ -2043,12 +2043,16 @@ cudaError_t inv_group_launch(const InverseArgs& a, const TemporalSet& ts, const 
   return cudaGetLastError();
 }
 
+// The staged form where it is built and a wait for its copies that ran out can
+// be told (a.err): without a flag, as in the allocation-free call, the form
+// that waits for nothing.
 template <int BW, int BH, int MODE>
 cudaError_t inv_group_mode(const InverseArgs& a, const TemporalSet& ts, const OlaFuse& of, cudaStream_t s) {
   if constexpr (run_staged<BW, BH, MODE>()) {
-    if (MODE < 2 || ts.count > 1) return inv_group_launch<BW, BH, MODE, true>(a, ts, of, s);
+    if (a.err && (MODE < 2 || ts.count > 1)) return inv_group_launch<BW, BH, MODE, true>(a, ts, of, s);
   }
-  if constexpr (MODE >= 2 || !run_staged<BW, BH, MODE>()) return inv_group_launch<BW, BH, MODE, false>(a, ts, of, s);
+  if constexpr (MODE != MODE_KALMAN || !run_staged<BW, BH, MODE>())  // (a Kalman filter's plane has a flag)
+    return inv_group_launch<BW, BH, MODE, false>(a, ts, of, s);
   return cudaErrorInvalidValue;
 }
 
