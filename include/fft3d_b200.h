@@ -171,9 +171,10 @@ int fft3d_plane_synchronize(fft3d_plane* h);
 /* Test hook (host-side fault injection, no counterpart in the reference): sets
  * the plane's device error flag to `bits`, as a kernel does when a bounded
  * wait runs out (bit 0: tensor-core MMA completion, bit 1: bulk copy
- * completion), after the work already queued for the plane. The next
- * host-buffer call, or fft3d_plane_synchronize, then reports the error and
- * clears the flag. Lets the device error path be tested without a real
+ * completion; where such waits feed overlap-adds of the same launch
+ * (NEO_FFT3D_FUSED_OLA=1) also what the launch leaves in its arrival counters),
+ * after the work already queued for the plane. The next host-buffer call, or
+ * fft3d_plane_synchronize, then reports the error and clears the flag. Lets the device error path be tested without a real
  * device fault. */
 int fft3d_plane_debug_set_error_flag(fft3d_plane* h, int bits);
 

@@ -1060,7 +1060,6 @@ int stage_pageable(fft3d_plane* P, fft3d_plane::Stage* sg, int n, const void* co
   return FFT3D_OK;
 }
 
-// Waits for a queued host-path call and reports a device error flag it saw.
 // Frames whose spectra a frame group n0 .. n0 + count - 1 needs at once.
 void group_range(const fft3d_plane* P, int n0, int count, int* lo, int* hi) {
   const int bt = std::max(P->ep.bt, 1);
@@ -1321,6 +1320,31 @@ int run_group(fft3d_plane* P, const fft3d::Deferred& d, cudaStream_t st) {
   return FFT3D_OK;
 }
 
+// The arrival counters back to zero, on the plane's stream after the work
+// queued there. A launch leaves them at zero unless some of its CTAs gave up (a
+// bounded wait that ran out), which leaves tiles counted in part: only the runs
+// of planes that fuse their overlap-adds (fuse_ola) wait for anything.
+cudaError_t clear_arrivals(fft3d_plane* P) {
+  if (!P->fuse_ola || !P->d_ola_cnt) return cudaSuccess;
+  return cudaMemsetAsync(P->d_ola_cnt, 0, (size_t)P->g.nblocks * sizeof(unsigned), P->stream);
+}
+
+// Clears the plane's error flag after a host-path call that saw it (P->mu not
+// held), and the counters that the failed launch may have left: calls queued
+// meanwhile ran on those, so they finish, and see the flag, first.
+void clear_error(fft3d_plane* P) {
+  if (P->fuse_ola) {
+    std::lock_guard<std::mutex> lk(P->mu);
+    if (P->last_work) cudaStreamWaitEvent(P->stream, P->last_work, 0);
+    clear_arrivals(P);
+    for (auto* st : {P->stream, P->s_down}) cudaStreamSynchronize(st);
+    cudaMemset(P->d_err, 0, sizeof(int));
+    return;
+  }
+  cudaMemset(P->d_err, 0, sizeof(int));
+}
+
+// Waits for a queued host-path call and reports a device error flag it saw.
 int finish_call(fft3d_plane* P, cudaEvent_t done, fft3d_plane::Stage* sg, bool learned) {
   const cudaError_t e = cudaEventSynchronize(done);
   give_sync_event(P, done);
@@ -1329,8 +1353,8 @@ int finish_call(fft3d_plane* P, cudaEvent_t done, fft3d_plane::Stage* sg, bool l
   for (int k = 0; k < 2; k++) {
     const int flag = flags[k];
     if (!flag) continue;
-    int* dflag = k == 0 ? P->d_err : (learned ? fft3d::psd::err_flag(P->psd_model) : nullptr);
-    if (dflag) cudaMemset(dflag, 0, sizeof(int));
+    if (k == 0) clear_error(P);
+    else if (learned) cudaMemset(fft3d::psd::err_flag(P->psd_model), 0, sizeof(int));
     return fail(FFT3D_E_CUDA, (flag & 4) ? "neo_fft3d: a bounds check of the checked build failed"
                               : (flag & 2) ? "neo_fft3d: bulk copy completion wait timed out"
                                            : "neo_fft3d: tensor-core MMA completion wait timed out");
@@ -1628,7 +1652,7 @@ int filter_group_host(fft3d_plane* P, int n0, int count, const void* const* src,
   if (e != cudaSuccess) return cuda_fail(e, "synchronize");
   if (gs->h_flags[0]) {
     const int flag = gs->h_flags[0];
-    cudaMemset(P->d_err, 0, sizeof(int));
+    clear_error(P);
     return fail(FFT3D_E_CUDA, (flag & 4) ? "neo_fft3d: a bounds check of the checked build failed"
                                          : "neo_fft3d: a bounded completion wait timed out");
   }
@@ -1891,6 +1915,7 @@ int fft3d_plane_reset(fft3d_plane* P) {
   // waits for it on its own stream; the host does not wait.
   if (P->last_work) CK(cudaStreamWaitEvent(P->stream, P->last_work, 0), "reset");
   for (auto& s : P->slots) { s.frame = -1; s.stamp = 0; }
+  CK(clear_arrivals(P), "counter reset");
   if (P->ep.bt == 0) {
     const size_t n = P->spec_elems();
     CK(cudaMemsetAsync(P->d_last, 0, n * sizeof(float2), P->stream), "Kalman reset");
@@ -2114,6 +2139,10 @@ int fft3d_plane_synchronize(fft3d_plane* P) {
                        "error flag");
   for (int k = 0; k < 2; k++) {
     if (!flags[k]) continue;
+    if (k == 0) {
+      CK(clear_arrivals(P), "counter reset");
+      CK(cudaStreamSynchronize(P->stream), "counter reset");
+    }
     CK(cudaMemset(k == 0 ? P->d_err : fft3d::psd::err_flag(P->psd_model), 0, sizeof(int)), "error flag");
     return fail(FFT3D_E_CUDA, (flags[k] & 4) ? "neo_fft3d: a bounds check of the checked build failed"
                               : (flags[k] & 2) ? "neo_fft3d: bulk copy completion wait timed out"
@@ -2130,6 +2159,13 @@ int fft3d_plane_debug_set_error_flag(fft3d_plane* P, int bits) {
   if (P->last_work) CK(cudaEventSynchronize(P->last_work), "synchronize");
   CK(cudaStreamSynchronize(P->stream), "synchronize");
   CK(cudaMemcpy(P->d_err, &bits, sizeof(int), cudaMemcpyHostToDevice), "error flag");
+  if ((bits & 2) && P->fuse_ola && P->d_ola_cnt) {
+    // ... with tiles counted in part, as CTAs that gave up leave them
+    const std::vector<unsigned> one((size_t)P->g.nblocks, 1u);
+    CK(cudaMemcpyAsync(P->d_ola_cnt, one.data(), one.size() * sizeof(unsigned), cudaMemcpyHostToDevice, P->stream),
+       "arrival counters");
+    CK(cudaStreamSynchronize(P->stream), "arrival counters");
+  }
   return FFT3D_OK;
 }
 
