@@ -1431,6 +1431,16 @@ int check_group_args(const fft3d_plane* P, int count, const void* const* src, co
   return FFT3D_OK;
 }
 
+// The row pitches of a frame whose crop borders are copied from source to output
+// plane: rows may not overlap (nor run backwards), as for any pitched copy.
+int check_border_pitches(const fft3d_plane* P, const void* src, int src_stride, int dst_stride) {
+  const fft3d_params& ep = P->ep;
+  if ((ep.l <= 0 && ep.t <= 0 && ep.r <= 0 && ep.b <= 0) || !src) return FFT3D_OK;
+  const int row = P->d.width * P->bytes;
+  if (src_stride < row || dst_stride < row) return cuda_fail(cudaErrorInvalidPitchValue, "plane copy");
+  return FFT3D_OK;
+}
+
 // Whether a call of `count` frames runs as a frame group: planes on the
 // default or the tensor-core path. Their new frames' forward transforms and
 // their overlap-adds run as one launch each; the filter/inverse runs as one
@@ -1983,7 +1993,9 @@ int fft3d_plane_filter_device(fft3d_plane* P, int n, const void* const src[5], c
   std::lock_guard<std::mutex> lk(P->mu);
   CK(cudaSetDevice(P->device), "cudaSetDevice");
   cudaStream_t st = stream ? (cudaStream_t)stream : P->stream;
-  const int rc = run_filter(P, n, src, src_stride, dst, dst_stride, false, st);
+  int rc = src ? check_border_pitches(P, src[2], src_stride[2], dst_stride) : FFT3D_OK;
+  if (rc) return rc;
+  rc = run_filter(P, n, src, src_stride, dst, dst_stride, false, st);
   mark_work(P, st);
   return rc;
 }
@@ -1995,6 +2007,8 @@ int fft3d_plane_filter_frames_device(fft3d_plane* P, int n0, int count, const vo
   std::lock_guard<std::mutex> lk(P->mu);
   CK(cudaSetDevice(P->device), "cudaSetDevice");
   cudaStream_t st = stream ? (cudaStream_t)stream : P->stream;
+  for (int j = 0; j < count; j++)
+    if ((rc = check_border_pitches(P, src[j + 2], src_stride[j + 2], dst_stride[j]))) return rc;
   rc = filter_group(P, n0, count, src, src_stride, dst, dst_stride, st);
   mark_work(P, st);
   return rc;
