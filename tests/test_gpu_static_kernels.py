@@ -42,3 +42,18 @@ def test_static_filter_waits_for_nothing(gpu, bw, bt):
     assert len(names) == 1, names
     staged = re.search(r"k_filter_inverse_group<\d+, \d+, -?\d+, (\w+)>", names[0])
     assert staged and staged.group(1) in ("false", "0"), names
+
+
+@pytest.mark.gpu
+def test_static_tables_of_small_blocks_go_up_in_less(gpu):
+    """Blocks up to 32 x 32 (the default) send their tables in the smaller set of
+    launch parameters, larger blocks in the large one."""
+    import torch
+    sent = {}
+    for bw, bh, ow in ((8, 8, 4), (16, 32, 8), (32, 32, 16), (32, 32, 0), (32, 48, 16), (48, 48, 24)):
+        names = [n for n in _kernels(torch, bt=1, bw=bw, bh=bh, ow=ow, oh=ow) if "k_static_tables" in n]
+        assert len(names) == 1, names
+        sent[bw, bh, ow] = int(re.search(r"k_static_tables<(\d+)>", names[0]).group(1))
+    small, large = sent[8, 8, 4], sent[48, 48, 24]
+    assert small < large
+    assert [sent[k] for k in ((16, 32, 8), (32, 32, 16), (32, 32, 0), (32, 48, 16))] == [small, small, small, large], sent
