@@ -186,8 +186,10 @@ int fft3d_plane_set_timing(fft3d_plane* h, int enable);
  * event milliseconds, out[3k+2] summed algorithmic bytes (what the launch's
  * interface must read and write once), for k = 0 forward (gather + window +
  * r2c), 1 filter + inverse (spectra in, time-domain blocks out), 2 overlap-add
- * (time-domain blocks in, pixels out), 3 fused (newest frame's pixels and the
- * older spectra in; newest spectrum and time-domain blocks out), 4 streaming
+ * (time-domain blocks in, pixels out), 3 one-launch
+ * frames (newest frame's pixels and the older spectra in; newest spectrum out,
+ * and pixels, or time-domain blocks where the overlap-add is a launch of its
+ * own; no counts of k = 0 and 1, nor then of 2), 4 streaming
  * filter (the window's spectra in, filtered spectrum out). Waits for the
  * recorded launches. */
 int fft3d_plane_timing(fft3d_plane* h, double out[15]);
@@ -213,7 +215,8 @@ int fft3d_plane_timing(fft3d_plane* h, double out[15]);
  * it from the host. Not for use across a cudaDeviceReset of a device it has
  * run on (the address and tables are kept per device for the process's life).
  * Output equals fft3d_plane_filter_device's with the same parameters, byte
- * for byte (the same kernels). */
+ * for byte (the same arithmetic; small planes of integer samples take one
+ * launch per frame there and four here). */
 int fft3d_filter2d_static(const fft3d_params* p, const fft3d_plane_desc* d, const void* src, int src_stride,
                           void* dst, int dst_stride, void* stream);
 

@@ -18,7 +18,8 @@ struct Deferred {
   struct Fwd { ForwardArgs a; int bytes; int plane; };
   struct Inv { InverseArgs a; int mode; int plane; };
   struct Ola { OlaArgs a; int bytes; int plane; };
-  // borders: only the crop borders are needed (the overlap-add writes the rest)
+  // borders: only the crop borders are needed (the overlap-add writes the rest).
+  // Frame groups copy just those; a batch step copies the whole plane.
   struct Copy { void* dst; size_t dpitch; const void* src; size_t spitch; size_t width; size_t height; int plane; bool borders; };
   // consecutive filter/inverse records of one plane and mode (a frame group's
   // run) merged into one work list: one CTA per block for all its frames

@@ -49,10 +49,21 @@ int cuda_fail(cudaError_t e, const char* what) {
   } while (0)
 
 // Most blocks of a plane whose frames go in one launch (k_frame): about three
-// CTAs per SM, one block each. One-frame calls, us per frame with one launch /
-// three, one plane and three planes on three streams: 48 x 48 blocks, 108
-// blocks 24 / 25 and 29 / 40, 374 blocks 27 / 27 and 40 / 40; 32 x 32 at bt = 5,
-// 336 blocks 19 / 23 and 25 / 40, 744 blocks 31 / 27 and 67 / 40.
+// CTAs per SM, one block each. One-frame calls queued one after another, us per
+// frame with three launches / one, bt = 3 (-1, 0, 1 and 5 are alike), each plane
+// on a stream of its own:
+//                        one plane    three such planes
+//   8 x 8    400 blocks  14.4 / 12.4  29 / 16
+//   16 x 16  400         16.5 / 14.4  30 / 17
+//   32 x 32  400         20.6 / 18.5  29 / 23
+//   48 x 48   64         23.7 / 22.6  30 / 26
+//   48 x 48  196         23.7 / 24.7  30 / 33
+//   48 x 48  400         25.6 / 26.6  36 / 39
+// and 4:2:0 clips of 640 x 480 with 48 x 48 blocks (374 and 108 blocks) 33 / 31, 57
+// / 49 when each frame is waited for. 48 x 48 blocks lose where many are in
+// flight: three planes of 196 blocks by 10 % (waited for they gain 8 %), and
+// chroma planes of 165 beside a luma plane of 588 on three launches 37 / 45. At
+// 744 blocks of 32 x 32, bt = 5, one launch loses: 27 / 31, three planes 40 / 67.
 constexpr int kOneLaunchBlocks = 450;
 
 struct Slot {

@@ -688,15 +688,6 @@ __host__ __device__ constexpr int win_lo() { return MODE >= 2 ? 2 - MODE / 2 : 2
 template <int MODE>
 __host__ __device__ constexpr int win_hi() { return MODE >= 2 ? 2 + (MODE - 1) / 2 : 2; }
 
-template <int MODE>
-__device__ __forceinline__ float2 filter_bin(const InverseArgs& a, size_t off, int bin, float gf, bool commit) {
-  float2 w[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++)
-    w[k] = (k >= win_lo<MODE>() && k <= win_hi<MODE>()) ? __ldg(a.in[k] + off + bin) : make_float2(0.f, 0.f);
-  return filter_vals<MODE>(a, w, off, bin, gf, bin_tab<MODE>(a, bin), commit);
-}
-
 // separate sharpen/dehalo pass on a filtered bin, src/code_impl/Sharpen.cpp:13-63
 // (the grid term removed and restored with packed f32x2 operations)
 __device__ __forceinline__ float2 sharpen_bin(const InverseArgs& a, float2 v, const BinTab& tb, float gf) {
@@ -1015,14 +1006,6 @@ __global__ void __launch_bounds__(256) k_filter_frames(InverseArgs a, const __gr
 template <int BW, int BH>
 __host__ __device__ constexpr int fft_ctas(int nblocks) {
   return (nblocks + kWarps * blocks_per_warp<BW>() - 1) / (kWarps * blocks_per_warp<BW>());
-}
-
-// A window-spectrum value, read once per CTA: not kept in L1, where the
-// per-bin tables (grid, wsharpen) that every chunk reads should stay.
-__device__ __forceinline__ float2 ld_stream(const float2* p) {
-  float2 v;
-  asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
-  return v;
 }
 
 // Where a CTA finds its window spectra and writes its time-domain blocks:
@@ -1358,8 +1341,9 @@ __device__ __forceinline__ void bulk_init(uint64_t* bar) {
 
 // Spectrum tiles one CTA of k_filter_inverse_group works on (blocks x frames
 // of the run): as many as its 128 threads have columns for in one round of
-// the column transforms, while 6 CTAs stay resident per SM (36 KB of tiles),
-// and at least the longest run's frames.
+// the column transforms, within 36 KB, and at least the longest run's frames
+// (staged runs add their window's extra ones, run_tiles; run_ctas says how many
+// CTAs then reside per SM).
 template <int BW, int BH>
 __host__ __device__ constexpr int group_tiles() {
   const int lanes = kWarps * 32 / (BW / 2), fit = 36 * 1024 / (BH * (BW / 2 + 1) * 8);
@@ -2021,8 +2005,8 @@ inline bool ola_fuse_ok(const OlaFuse& of, const Geom& g) {
 
 // Blocks per CTA of a run whose block takes `count` tiles, over nblocks
 // blocks: as many as the CTA has tiles for, but no more than keep every CTA
-// slot of the chip filled (6 per SM), down to one block per CTA for small
-// planes.
+// slot of the chip filled (run_ctas per SM), down to one block per CTA for
+// small planes.
 template <int BW, int BH, int MODE, bool STAGED>
 int group_blocks_per_cta(int nblocks, int count) {
   const int most = std::max(1, run_tiles<BW, BH, MODE, STAGED>() / count);

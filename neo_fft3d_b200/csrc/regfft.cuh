@@ -19,7 +19,7 @@ namespace fft3d {
 // (each lane rounds like the scalar operation). Held as one 64-bit value and
 // worked on with PTX: the same arithmetic on float2 and its intrinsics cost 50
 // register moves per bin pair and frame at bt = 5 (188 instructions instead of
-// 128), because the halves are then allocated one by one.
+// 131), because the halves are then allocated one by one.
 using f2x = unsigned long long;
 __device__ __forceinline__ f2x pk2(float lo, float hi) {
   f2x r;
