@@ -51,7 +51,10 @@ def device_fps(noisy, model, pooled, reps=3):
     eng = engine.PlaneEngine(p, d)
     if model is not None:
         eng.set_psd(model, pooled)
-    s = torch.cuda.current_stream()
+    # (a stream of its own: on the default one, whose handle is 0, the engine
+    # would take the plane's stream, and the events below would time the host)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
 
     def run():
         eng.reset()
