@@ -176,8 +176,10 @@ __device__ __forceinline__ const T* fwd_row_src(const ForwardArgs& a, const Win&
 }
 
 // Row y of block `blk`: gather (mirrored at the plane edges), analysis window,
-// r2c along x into row y of Sb.
-template <int BW, int BH, typename T, class Win>
+// r2c along x into row y of Sb. PARAM: the window along x comes as halves from
+// the launch parameters, else from memory (a power of two leaves the products
+// the same).
+template <int BW, int BH, typename T, bool PARAM, class Win>
 __device__ __forceinline__ void fwd_row(const ForwardArgs& a, const Win& win, int blk, int y, float2* Sb) {
   constexpr int NH = BW / 2 + 1;
   const Geom& g = a.g;
@@ -198,9 +200,9 @@ __device__ __forceinline__ void fwd_row(const ForwardArgs& a, const Win& win, in
       r[x] = (row_ok && FFT3D_IN(xi >= 0 && xi < g.W, a.err)) ? load_sample<T>(srow + xi) - a.base : 0.f;
     }
   }
-  const float wy = __ldg(a.wan_y + y);
+  const float wy = __ldg(a.wan_y + y) * (PARAM ? 2.f : 1.f);
 #pragma unroll
-  for (int x = 0; x < BW; x++) r[x] = r[x] * __ldg(a.wan_x + x) * wy;
+  for (int x = 0; x < BW; x++) r[x] = r[x] * (PARAM ? a.wx_half[x].x : __ldg(a.wan_x + x)) * wy;
   float2 c[NH];
   rfft<BW>(r, c);
   float2* row = Sb + y * NH;
@@ -307,7 +309,7 @@ __device__ __forceinline__ void frame_forward(const ForwardArgs& a, int blk0, in
   const int t = threadIdx.x;
   for (int i = t; i < count * BH; i += NT) {
     const int b = i / BH;
-    fwd_row<BW, BH, T>(a, win, blk0 + b, i - b * BH, S + b * BINS);
+    fwd_row<BW, BH, T, false>(a, win, blk0 + b, i - b * BH, S + b * BINS);
   }
   __syncthreads();
   for (int i = t; i < count * HC; i += NT) {
@@ -329,9 +331,19 @@ template <int BW>
 __host__ __device__ constexpr int fwd_blocks() { return kWarps * blocks_per_warp<BW>(); }
 template <int BW>
 __host__ __device__ constexpr int fwd_threads() { return fwd_blocks<BW>() * (BW / 2); }
+// Whether a thread takes two rows at once, or one: pairs, unless a block has so
+// few rows that its pairs fill half the threads or less, or two thirds where two
+// rows of 48 samples take the registers of more than 96 a thread. us per frame
+// with pairs / single rows: 32 x 16, 800 blocks 10.2 / 8.7, 16000 blocks 21.7 /
+// 18.9; 48 x 16, 16000 blocks 38.6 / 30.5; 48 x 32, 3600 blocks 21.2 / 19.1, 16000
+// blocks 50.2 / 45.5; 24 x 16, 1600 blocks 9.3 / 10.6, 16000 blocks 18.9 / 18.6; 32 x
+// 32, 8000 blocks 20.7 / 21.4.
+template <int BW, int BH>
+__host__ __device__ constexpr bool fwd_pairs() { return BH * 4 > BW * (BW > 32 ? 3 : 2); }
 
 // Forward transform of fwd_blocks<BW>() consecutive blocks per CTA.
-//  rows: a thread takes rows y and y + bh/2 of a block at once, packed
+//  rows: a thread takes one row, or (fwd_pairs) rows y and y + bh/2 of a block at
+//   once, packed
 //   (rfft_pair): gather with mirrored edges, analysis window, r2c; their
 //   spectra go to shared memory interleaved, 16 bytes per bin {A.re, B.re,
 //   A.im, B.im};
@@ -347,7 +359,8 @@ __host__ __device__ constexpr int fwd_threads() { return fwd_blocks<BW>() * (BW 
 template <int BW, int BH, typename T, class Win>
 __device__ __forceinline__ void forward_blocks(const ForwardArgs& a, int cta, const Win& win) {
   constexpr int NH = BW / 2 + 1, HC = BW / 2, HB = BH / 2, BINS = BH * NH, NT = fwd_threads<BW>();
-  constexpr bool WARP = HB == HC && 32 % HC == 0;  // a block's work stays in one warp
+  constexpr bool PAIRS = fwd_pairs<BW, BH>();
+  constexpr bool WARP = (PAIRS ? HB : BH) == HC && 32 % HC == 0;  // a block's work stays in one warp
   constexpr int GT = WARP ? 32 : NT, GB = GT / HC;  // threads and blocks of a group that synchronises
   constexpr int WORDS = BW * (int)sizeof(T) / 4;
   extern __shared__ __align__(16) float2 smem2[];
@@ -361,7 +374,12 @@ __device__ __forceinline__ void forward_blocks(const ForwardArgs& a, int cta, co
     else __syncthreads();
   };
   if (WARP && nvalid <= 0) return;
-  for (int i = t; i < GB * HB; i += GT) {
+  if constexpr (!PAIRS)
+    for (int i = t; i < GB * BH; i += GT) {
+      const int b = i / BH;
+      if (b < nvalid) fwd_row<BW, BH, T, true>(a, win, blk0 + b, i - b * BH, S + b * BINS);
+    }
+  for (int i = t; PAIRS && i < GB * HB; i += GT) {
     const int b = i / HB, y = i - b * HB;
     if (b >= nvalid) continue;
     float4* quads = reinterpret_cast<float4*>(S + b * BINS) + y * NH;
@@ -409,34 +427,38 @@ __device__ __forceinline__ void forward_blocks(const ForwardArgs& a, int cta, co
   const int cb = t / HC, c = t - cb * HC;
   const bool mine = cb < nvalid;
   float2* Sb = S + cb * BINS;
-  if (mine) {
-    const float4* quads = reinterpret_cast<const float4*>(Sb);
+  if constexpr (!PAIRS) {
+    if (mine) fwd_col<BW, BH>(Sb, c);
+  } else {
+    if (mine) {
+      const float4* quads = reinterpret_cast<const float4*>(Sb);
 #pragma unroll
-    for (int y = 0; y < HB; y++) {
-      const float4 q = quads[y * NH + c];
-      col[y] = make_float2(q.x, q.z);
-      col[y + HB] = make_float2(q.y, q.w);
-      if (c == 0) {  // real columns 0 and bw/2 as one complex sequence
-        const float4 n = quads[y * NH + HC];
-        col[y].y = n.x;
-        col[y + HB].y = n.y;
+      for (int y = 0; y < HB; y++) {
+        const float4 q = quads[y * NH + c];
+        col[y] = make_float2(q.x, q.z);
+        col[y + HB] = make_float2(q.y, q.w);
+        if (c == 0) {  // real columns 0 and bw/2 as one complex sequence
+          const float4 n = quads[y * NH + HC];
+          col[y].y = n.x;
+          col[y + HB].y = n.y;
+        }
       }
     }
-  }
-  sync();
-  if (mine) {
-    cfft<BH, -1>(col);
-    if (c == 0) {
+    sync();
+    if (mine) {
+      cfft<BH, -1>(col);
+      if (c == 0) {
 #pragma unroll
-      for (int h = 0; h < BH; h++) {
-        const float2 zh = col[h], zm = cconj(col[(BH - h) % BH]);
-        Sb[h * NH] = make_float2(0.5f * (zh.x + zm.x), 0.5f * (zh.y + zm.y));
-        const float2 d = csub(zh, zm);
-        Sb[h * NH + HC] = make_float2(0.5f * d.y, -0.5f * d.x);
+        for (int h = 0; h < BH; h++) {
+          const float2 zh = col[h], zm = cconj(col[(BH - h) % BH]);
+          Sb[h * NH] = make_float2(0.5f * (zh.x + zm.x), 0.5f * (zh.y + zm.y));
+          const float2 d = csub(zh, zm);
+          Sb[h * NH + HC] = make_float2(0.5f * d.y, -0.5f * d.x);
+        }
+      } else {
+#pragma unroll
+        for (int h = 0; h < BH; h++) Sb[h * NH + c] = col[h];
       }
-    } else {
-#pragma unroll
-      for (int h = 0; h < BH; h++) Sb[h * NH + c] = col[h];
     }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
