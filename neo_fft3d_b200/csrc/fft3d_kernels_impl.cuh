@@ -1015,13 +1015,68 @@ __global__ void __launch_bounds__(256) k_filter_frames(InverseArgs a, const __gr
   }
 }
 
+// The Kalman state of two neighbouring bins: filtered values, covariances,
+// process covariances (loads that do not allocate in L1: each is read once and
+// written back by this thread).
+struct KalmanPair {
+  float4 l;
+  float2 cv, cp;
+  __device__ __forceinline__ void load(const InverseArgs& a, size_t at) {
+    asm("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+        : "=f"(l.x), "=f"(l.y), "=f"(l.z), "=f"(l.w) : "l"(a.kal_last + at));
+    asm("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(cv.x), "=f"(cv.y) : "l"(a.kal_covar + at));
+    asm("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(cp.x), "=f"(cp.y) : "l"(a.kal_covarp + at));
+  }
+  // (a load that the compiler keeps before the stores that follow)
+  __device__ __forceinline__ void load_before_stores(const InverseArgs& a, size_t at) {
+    l = *reinterpret_cast<const float4*>(a.kal_last + at);
+    cv = *reinterpret_cast<const float2*>(a.kal_covar + at);
+    cp = *reinterpret_cast<const float2*>(a.kal_covarp + at);
+  }
+  __device__ __forceinline__ void store(const InverseArgs& a, size_t at) const {
+    *reinterpret_cast<float4*>(a.kal_last + at) = l;
+    *reinterpret_cast<float2*>(a.kal_covar + at) = cv;
+    *reinterpret_cast<float2*>(a.kal_covarp + at) = cp;
+  }
+  // One frame's values of the pair (bins bin, bin + 1 of the block at `off`): the filtered ones.
+  __device__ __forceinline__ float4 step(const InverseArgs& a, const float4& c, size_t off, int bin) {
+    float s0 = a.c.sigma2n_2d, s1 = a.c.sigma2n_2d;
+    if (a.psd) {
+      s0 = fmaxf(learned_noise(a, off, bin), 1e-15f);
+      s1 = fmaxf(learned_noise(a, off, bin + 1), 1e-15f);
+    } else if (a.c.pattern) {
+      s0 = fmaxf(__ldg(a.t.pattern2d + bin), 1e-15f);
+      s1 = fmaxf(__ldg(a.t.pattern2d + bin + 1), 1e-15f);
+    }
+    float2 l0 = make_float2(l.x, l.y), l1 = make_float2(l.z, l.w);
+    kalman_step(a, make_float2(c.x, c.y), s0, l0, cv.x, cp.x);
+    kalman_step(a, make_float2(c.z, c.w), s1, l1, cv.y, cp.y);
+    l = make_float4(l0.x, l0.y, l1.x, l1.y);
+    return l;
+  }
+};
+
+// A thread's walk over the bin pairs of consecutive blocks, `STEP` pairs at a
+// time: block b and first bin, kept without divisions.
+template <int BINS, int STEP>
+struct PairCursor {
+  int b, bin;
+  __device__ __forceinline__ explicit PairCursor(int pair) : b(pair / (BINS / 2)), bin(2 * (pair % (BINS / 2))) {}
+  __device__ __forceinline__ void step() {
+    b += 2 * STEP / BINS;
+    bin += 2 * STEP % BINS;
+    if (bin >= BINS) bin -= BINS, b++;
+  }
+};
+
 // ---------------------------------------------------------------- inverse
 
 // One warp filters and inverse-transforms blocks_per_warp<BW>() blocks:
-//  A. every bin of a block, consecutive bin pairs on consecutive lanes
-//     (coalesced 16-byte loads of the bt spectra), through the filter and the
-//     separate sharpen/dehalo pass (whose grid fraction is the filtered DC,
-//     lane 0's first bin); results to shared memory;
+//  A. every bin, consecutive bin pairs on consecutive lanes (coalesced 16-byte
+//     loads of the bt spectra), through the filter and the separate
+//     sharpen/dehalo pass (whose grid fraction is the filtered DC); results to
+//     shared memory. Block by block, or the warp's blocks as one stream
+//     (stream_blocks);
 //  B. one column per lane: inverse complex DFT along y (DC and Nyquist columns
 //     together: both are Hermitian, so their inverses are real);
 //  C. one row per lane: c2r along x, 16-byte stores of the time-domain rows.
@@ -1045,10 +1100,22 @@ struct FrameWin {
   __device__ __forceinline__ float* tdom() const { return t; }
 };
 
+// Blocks that a warp filters as one stream: all its blocks where single blocks
+// leave many lanes idle in their last round (16 x 16: 72 pairs are three rounds,
+// four blocks' 288 are nine), more of them for a window of 2 to 4 frames, whose
+// rounds the stream's block index and shuffles cost more. us per frame block by
+// block / as a stream: 16 x 16, 16000 blocks, bt = 5 35 / 31, bt = 1 22 / 19, bt = 3
+// 25.7 / 25.9; 24 x 16, 30000 blocks, bt = 5 78 / 67, bt = 3 55 / 56, bt = 2 41 / 50.
+template <int BW, int BH, int MODE>
+__host__ __device__ constexpr int stream_blocks() {
+  constexpr int PAIRS = BH * (BW / 2 + 1) / 2, LANES = (PAIRS + 31) / 32 * 32;
+  constexpr int percent = MODE == 2 || MODE == 3 ? 65 : (MODE == 4 ? 76 : 87);
+  return 100 * PAIRS < percent * LANES ? blocks_per_warp<BW>() : 1;
+}
+
 template <int BW, int BH, int MODE, class Win>
 __device__ __forceinline__ void filter_inverse_cta_w(const InverseArgs& a, int vcta, const Win& win) {
-  constexpr int NH = BW / 2 + 1, HC = BW / 2, NBW = blocks_per_warp<BW>(), BINS = BH * NH;
-  constexpr int PER = (BINS / 2 + 31) / 32;
+  constexpr int NH = BW / 2 + 1, HC = BW / 2, NBW = blocks_per_warp<BW>(), BINS = BH * NH, PAIRS = BINS / 2;
   extern __shared__ __align__(16) float2 smem2[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* S = smem2 + warp * NBW * BINS;
@@ -1058,63 +1125,96 @@ __device__ __forceinline__ void filter_inverse_cta_w(const InverseArgs& a, int v
   if (blk0 >= g.nblocks) return;
   const float gs0 = __ldg(&a.t.grid[0].x);
   constexpr int LO = win_lo<MODE>(), HI = win_hi<MODE>(), NW = HI - LO + 1;
-  // load-pipeline depth (chunks of 32 bin pairs in flight), fewer as the
-  // window (and the registers per chunk) grows
-  constexpr int DW = NW <= 1 ? 4 : (NW == 2 ? 4 : (NW == 3 ? 3 : 2));
-  constexpr int D = PER < DW ? PER : DW;
+  // load-pipeline depth (rounds of 32 bin pairs in flight), fewer as the
+  // window (and the registers per round) grows
+  constexpr int GROUP = stream_blocks<BW, BH, MODE>();
+  constexpr int ROUNDS = (GROUP * PAIRS + 31) / 32;
+  constexpr int DW = NW <= 1 ? (MODE == MODE_KALMAN ? 3 : 4) : (NW == 2 ? 4 : (NW == 3 ? 3 : 2));
+  constexpr int D = ROUNDS < DW ? ROUNDS : DW;
 #pragma unroll 1
-  for (int b = 0; b < NBW; b++) {
-    const int blk = blk0 + b;
-    if (blk >= g.nblocks) break;
-    const size_t off = (size_t)blk * BINS;
-    float gf = 0.f;
-    if constexpr (MODE >= 1) gf = a.c.degrid * __ldg(&win.in(2)[off].x) / gs0;
-    // software pipeline: the window's values of chunk j + D are loaded while
-    // chunk j is filtered, so D x NW loads per lane are always in flight
-    float4 buf[D][NW];
-    auto load = [&](int j, float4(&dst)[NW]) {
-      const int i = 2 * (lane + 32 * j);
+  for (int b0 = 0; b0 < NBW; b0 += GROUP) {
+    if (blk0 + b0 >= g.nblocks) break;
+    const size_t off0 = (size_t)(blk0 + b0) * BINS;
+    const int pairs = GROUP == 1 ? PAIRS : min(GROUP, g.nblocks - blk0 - b0) * PAIRS;
+    const int rounds = GROUP == 1 ? ROUNDS : (pairs + 31) / 32;
+    auto fetch = [&](int q, float4(&dst)[NW]) {  // the window of pair q
 #pragma unroll
       for (int k = 0; k < NW; k++)
-        dst[k] = (i < BINS && FFT3D_IN(win.in(LO + k) != nullptr && off + i + 1 < (size_t)g.nblocks * BINS, a.err))
-                     ? ld_stream4(win.in(LO + k) + off + i)
+        dst[k] = (q < pairs && FFT3D_IN(win.in(LO + k) != nullptr && off0 + 2 * q + 1 < (size_t)g.nblocks * BINS, a.err))
+                     ? ld_stream4(win.in(LO + k) + off0 + 2 * q)
                      : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-#pragma unroll
-    for (int j = 0; j < D; j++) load(j, buf[j]);
-    float gsh = 0.f;
-    // (D chunks to a turn of the loop: the whole block unrolled is four times
-    // the code, and its instruction-cache misses cost more than the loop)
-#pragma unroll 1
-    for (int j0 = 0; j0 < PER; j0 += D) {
-#pragma unroll
-      for (int u = 0; u < D; u++) {
-        const int j = j0 + u, i = 2 * (lane + 32 * j);
-        if (j >= PER) break;
-        const bool in = i < BINS;
+    auto filter = [&](const float4(&in)[NW], KalmanPair& state, size_t off, int bin, float gf) {
+      if constexpr (MODE == MODE_KALMAN) {
+        return state.step(a, in[0], off, bin);
+      } else {
         float4 w[5];
 #pragma unroll
-        for (int k = 0; k < 5; k++) w[k] = (k >= LO && k < LO + NW) ? buf[u][k - LO] : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (j + D < PER) load(j + D, buf[u]);
+        for (int k = 0; k < 5; k++) w[k] = (k >= LO && k < LO + NW) ? in[k - LO] : make_float4(0.f, 0.f, 0.f, 0.f);
+        return group_filter_one<MODE>(a, off, bin, w, gf);
+      }
+    };
+    // software pipeline: the window (and Kalman state) of round j + D is loaded
+    // while round j is filtered, so D x NW loads per lane are always in flight
+    float4 buf[D][NW];
+    KalmanPair kal[MODE == MODE_KALMAN ? D : 1];
+#pragma unroll
+    for (int j = 0; j < D; j++) {
+      fetch(lane + 32 * j, buf[j]);
+      if (MODE == MODE_KALMAN && lane + 32 * j < pairs) kal[j].load(a, off0 + 2 * (lane + 32 * j));
+    }
+    // grid fractions of the block's DC and of its filtered DC: lane b's are block b0 + b's
+    float gf_mine = 0.f, gsh_mine = 0.f;
+    if (lane * PAIRS < pairs) {
+      if constexpr (MODE >= 1) gf_mine = a.c.degrid * __ldg(&win.in(2)[off0 + lane * BINS].x) / gs0;
+      if (GROUP > 1 && a.c.do_sharpen) {
+        float4 dc[NW];
+        fetch(lane * PAIRS, dc);
+        KalmanPair state;
+        if constexpr (MODE == MODE_KALMAN) state.load_before_stores(a, off0 + lane * BINS);
+        gsh_mine = a.c.degrid * filter(dc, state, off0 + lane * BINS, 0, gf_mine).x / gs0;
+      }
+    }
+    float gf = MODE >= 1 ? __shfl_sync(0xffffffffu, gf_mine, 0) : 0.f, gsh = 0.f;
+    PairCursor<BINS, 32> at(lane);
+    // (D rounds to a turn of the loop: all of it unrolled is many times the
+    // code, and its instruction-cache misses cost more than the loop)
+#pragma unroll 1
+    for (int j0 = 0; j0 < rounds; j0 += D) {
+#pragma unroll
+      for (int u = 0; u < D; u++) {
+        const int j = j0 + u, q = lane + 32 * j;
+        if (j >= rounds) break;
+        const bool in = q < pairs;
+        const int bin = GROUP == 1 ? 2 * q : at.bin;
+        const size_t off = GROUP == 1 ? off0 : off0 + at.b * BINS;
+        if constexpr (GROUP > 1) {
+          if (MODE >= 1) gf = __shfl_sync(0xffffffffu, gf_mine, at.b);
+          if (a.c.do_sharpen) gsh = __shfl_sync(0xffffffffu, gsh_mine, at.b);
+          at.step();
+        }
+        float4 w[NW];
+#pragma unroll
+        for (int k = 0; k < NW; k++) w[k] = buf[u][k];
+        KalmanPair state;
+        if constexpr (MODE == MODE_KALMAN) state = kal[u];
+        if (j + D < rounds) {
+          fetch(q + 32 * D, buf[u]);
+          if (MODE == MODE_KALMAN && q + 32 * D < pairs) kal[u].load(a, off0 + 2 * (q + 32 * D));
+        }
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (in) {
-          if constexpr (MODE == MODE_KALMAN) {
-            const float2 w0[5] = {{}, {}, {w[2].x, w[2].y}, {}, {}}, w1[5] = {{}, {}, {w[2].z, w[2].w}, {}, {}};
-            const float2 v0 = filter_vals<MODE>(a, w0, off, i, gf, BinTab{}, true);
-            const float2 v1 = filter_vals<MODE>(a, w1, off, i + 1, gf, BinTab{}, true);
-            v = make_float4(v0.x, v0.y, v1.x, v1.y);
-          } else {
-            v = group_filter_one<MODE>(a, off, i, w, gf);
-          }
+          v = filter(w, state, off, bin, gf);
+          if constexpr (MODE == MODE_KALMAN) state.store(a, off0 + 2 * q);
         }
         if (a.c.do_sharpen) {
-          // grid fraction of the sharpen pass: the filtered DC (lane 0, chunk 0)
-          if (j == 0) gsh = a.c.degrid * __shfl_sync(0xffffffffu, v.x, 0) / gs0;
+          // one block's filtered DC is lane 0's first bin
+          if (GROUP == 1 && j == 0) gsh = a.c.degrid * __shfl_sync(0xffffffffu, v.x, 0) / gs0;
           if (in)
-            v = bins_of(sharpen_pair(a, pair_of(v), pair_grid(a, i), pair_weights(a.t.wsharpen, a.c.use_sharpen, i),
-                                     pair_weights(a.t.wdehalo, a.c.use_dehalo, i), gsh));
+            v = bins_of(sharpen_pair(a, pair_of(v), pair_grid(a, bin), pair_weights(a.t.wsharpen, a.c.use_sharpen, bin),
+                                     pair_weights(a.t.wdehalo, a.c.use_dehalo, bin), gsh));
         }
-        if (in) *reinterpret_cast<float4*>(S + b * BINS + i) = v;
+        if (in) *reinterpret_cast<float4*>(S + b0 * BINS + 2 * q) = v;
       }
     }
   }
@@ -1164,8 +1264,15 @@ __global__ void __launch_bounds__(kWarps * 32) k_filter_inverse_frames(InverseAr
   filter_inverse_cta_w<BW, BH, MODE, FrameWin>(a, c, w);
 }
 
+// CTAs per SM of k_filter_inverse: 6 at 80 registers where that spills little
+// (24 x 16 blocks, bt = 2, 16000 of them: 29 us at 5, 24 at 6; 32 x 32, bt = 3, 8000:
+// 39 at 5, 52 at 6).
+template <int BH, int MODE>
+__host__ __device__ constexpr int inv_ctas() { return (MODE == 2 || MODE == 3) && BH <= 16 ? 6 : 5; }
+
 template <int BW, int BH, int MODE>
-__global__ void __launch_bounds__(kWarps * 32, ctas_for(5, kWarps * fft_smem_bytes<BW, BH>())) k_filter_inverse(InverseArgs a) {
+__global__ void __launch_bounds__(kWarps * 32, ctas_for(inv_ctas<BH, MODE>(), kWarps * fft_smem_bytes<BW, BH>()))
+    k_filter_inverse(InverseArgs a) {
   filter_inverse_cta<BW, BH, MODE>(a, blockIdx.x);
 }
 
@@ -1482,19 +1589,6 @@ __device__ __noinline__ void group_ola_tile(const OlaFuse& of, const TemporalSet
   else if (of.px == 2) group_ola_tile_v<T, 2>(of, ts, count, tx, ty);
   else group_ola_tile_v<T, 1>(of, ts, count, tx, ty);
 }
-
-// A thread's walk over the bin pairs of consecutive blocks, `STEP` pairs at a
-// time: block b and first bin, kept without divisions.
-template <int BINS, int STEP>
-struct PairCursor {
-  int b, bin;
-  __device__ __forceinline__ explicit PairCursor(int pair) : b(pair / (BINS / 2)), bin(2 * (pair % (BINS / 2))) {}
-  __device__ __forceinline__ void step() {
-    b += 2 * STEP / BINS;
-    bin += 2 * STEP % BINS;
-    if (bin >= BINS) bin -= BINS, b++;
-  }
-};
 
 // Window spectra beyond the run's own frames that a staged run keeps in shared memory.
 template <int MODE>
@@ -2062,16 +2156,24 @@ cudaError_t inv_group_mode(const InverseArgs& a, const TemporalSet& ts, const Ol
   return cudaErrorInvalidValue;
 }
 
-// One output frame of a Wiener 3D plane: large planes by k_filter_inverse (a
-// warp owns its blocks; no barriers, 2 x MODE loads in flight per lane), small
-// ones by k_filter_inverse_group with a CTA per block or two, which fills the
-// chip with fewer blocks and has a quarter of the serial work per thread.
-// Measured at bt = 5, 32 x 32 blocks, one stream: 8349 blocks 58 us by warps,
-// 67 us by CTAs; 2135 blocks 30 us and 27 us. Wiener 2D, Kalman and
-// sharpen-only frames read one spectrum, which a bulk copy brings in: by CTAs
-// at every size (8349 blocks at bt = 1: 43 us, 55 us by warps).
-template <int MODE>
-bool one_frame_by_warps(int nblocks) { return MODE >= 2 && nblocks > 4000; }
+// One output frame: many blocks by k_filter_inverse (a warp owns its blocks; no
+// barriers, the loads of 2 to 4 rounds in flight per lane), few by
+// k_filter_inverse_group with a CTA per block or more, which fills the chip with
+// fewer blocks and has a quarter of the serial work per thread. The line lies
+// where both take as long, us by CTAs / by warps: at 8 x 8, 800 blocks 10.6 / 8.6
+// (450 equal); wide blocks, whose few rows leave a CTA's threads idle: 32 x 16, 800
+// blocks 12.7 / 12.3, 3600 blocks 17.7 / 14.9; tall ones, whose columns are a warp's
+// longer chains: 16 x 32, 3600 blocks 18.9 / 19.4, 24 x 32, 2400 blocks 18.8 / 18.0;
+// 32 x 32 at bt = 3, 1600 blocks 18.6 / 17.8, at bt = 5, 2400 blocks 25.0 / 24.9, 3600
+// blocks 31.1 / 27.5. 48 x 48 at bt = 1 or -1 has one spectrum to read, by a bulk
+// copy, and the tiles of four resident CTAs: 8000 blocks 62 / 68. Kalman: 32 x 32,
+// 8000 blocks 51 / 37.
+template <int BW, int BH, int MODE>
+bool one_frame_by_warps(int nblocks) {
+  if (BW * BH >= 48 * 48 && (MODE == MODE_WIENER2D || MODE == MODE_SHARPEN_ONLY)) return false;
+  constexpr int square = MODE >= 4 ? 3000 : 1500;
+  return nblocks > (BW < 12 ? 400 : BW > BH ? 700 : BW == BH ? square : BW < 24 ? 4000 : 2000);
+}
 
 template <int BW, int BH, int MODE>
 cudaError_t inv_mode(const InverseArgs& a, cudaStream_t s) {
@@ -2089,14 +2191,12 @@ cudaError_t inv_mode(const InverseArgs& a, cudaStream_t s) {
     k_filter_inverse_bulk<BW, BH, MODE><<<grid, kBulkWarps * 32, bulk_smem, s>>>(a);
     return cudaGetLastError();
   }
-  if constexpr (MODE >= 2) {
-    if (one_frame_by_warps<MODE>(a.g.nblocks)) {
-      const int smem = kWarps * fft_smem_bytes<BW, BH>();
-      cudaError_t e = fft3d::smem_attr(k_filter_inverse<BW, BH, MODE>, smem);
-      if (e != cudaSuccess) return e;
-      k_filter_inverse<BW, BH, MODE><<<fft_grid<BW, BH>(a.g.nblocks), kWarps * 32, smem, s>>>(a);
-      return cudaGetLastError();
-    }
+  if (one_frame_by_warps<BW, BH, MODE>(a.g.nblocks)) {
+    const int smem = kWarps * fft_smem_bytes<BW, BH>();
+    cudaError_t e = fft3d::smem_attr(k_filter_inverse<BW, BH, MODE>, smem);
+    if (e != cudaSuccess) return e;
+    k_filter_inverse<BW, BH, MODE><<<fft_grid<BW, BH>(a.g.nblocks), kWarps * 32, smem, s>>>(a);
+    return cudaGetLastError();
   }
   // one frame is a run of one
   TemporalSet ts{};
