@@ -65,6 +65,15 @@ int cuda_fail(cudaError_t e, const char* what) {
 // chroma planes of 165 beside a luma plane of 588 on three launches 37 / 45. At
 // 744 blocks of 32 x 32, bt = 5, one launch loses: 27 / 31, three planes 40 / 67.
 constexpr int kOneLaunchBlocks = 450;
+// Most overlap-add items (adjacent pixels that go out together) of an output
+// tile in such a launch: the CTA that does the tile pays its reads' latency, 2.5
+// us, for every 128 of them, so twice to four times as many by the block's size.
+// One plane of 256 blocks, three launches / one: 32 x 32, overlap 16, 64 items 20.4 /
+// 17.3, overlap 10 and an odd width, 484 items 20.4 / 25.9 (with three planes in
+// flight 40 / 27: three launches are bound by their host); 48 x 48, overlap 16, 256
+// items 23.5 / 24.8, overlap 24 and an odd width, 576 items 25.0 / 38.1; 24 x 24,
+// overlap 2, 242 items 17.0 / 18.2, and an odd width, 484 items 17.0 / 22.4.
+int one_launch_items(const Geom& g) { return std::min(512, std::max(256, g.bw * g.bh / 2)); }
 
 struct Slot {
   float2* spec = nullptr;
@@ -874,7 +883,23 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
   const int newest = n + to;
   // Small planes (device calls, one frame at a time) do the whole frame in one
   // launch, the overlap-add too.
-  const bool small = P->path == 1 && !host && !g_defer && !P->bulk && P->g.nblocks <= kOneLaunchBlocks;
+  bool small = P->path == 1 && !host && !g_defer && !P->bulk && P->g.nblocks <= kOneLaunchBlocks && P->bytes != 4 &&
+               !learned;
+  float* tdom = P->occ > 0 ? P->tdom_extra[P->occ - 1] : P->d_tdom;
+  const float base = (P->bytes != 4 && P->d.is_chroma) ? (float)(1 << (P->d.bits - 1)) : 0.f;
+  fft3d::OlaFuse of{};
+  if (small) {
+    of.o = ola_args(P, nullptr, P->tab, base, dst, dst_stride);
+    fft3d::OlaFrameSet fs{};
+    fs.count = 1;
+    fs.tdom[0] = tdom;
+    of.dst[0] = fs.dst[0] = of.o.dst;
+    of.dst_stride[0] = fs.dst_stride[0] = dst_stride;
+    of.bytes = P->bytes;
+    of.px = fft3d::overlap_add_pixels(of.o, fs, P->bytes);
+    of.o.dst = nullptr;
+    small = P->g.sx * P->g.sy <= one_launch_items(P->g) * of.px;
+  }
   const bool fused = (P->path == 2 || small) && P->bytes != 4 && !learned && !find_slot(P, newest);
   bool ola_done = false;
   for (int d = from; d <= (fused ? to - 1 : to); d++) {
@@ -935,7 +960,6 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
   ia.kal_last = P->d_last;
   ia.kal_covar = P->d_cov;
   ia.kal_covarp = P->d_covp;
-  float* tdom = P->occ > 0 ? P->tdom_extra[P->occ - 1] : P->d_tdom;
   ia.tdom = tdom;
   ia.err = P->d_err;
   ia.bulk = (P->path == 1 || P->path == 3) ? P->bulk : 0;
@@ -951,23 +975,12 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
       fft3d::FrameArgs fa;
       fa.f = forward_args(P, new_src, new_stride, news->spec);
       fa.v = ia;
-      fa.of = fft3d::OlaFuse{};
       // (a frame filtered in place keeps its overlap-add as a launch of its
       // own: the arrivals order a tile after the blocks that make it, not after
       // the blocks that still read its pixels for their transforms, such as
       // those mirrored at the plane's edges)
-      if (small && !planes_meet(P, dst, dst_stride, new_src, new_stride) && ola_fuse_setup(P, &fa.of)) {
-        fa.of.o = ola_args(P, nullptr, P->tab, fa.f.base, dst, dst_stride);
-        fft3d::OlaFrameSet fs{};
-        fs.count = 1;
-        fs.tdom[0] = tdom;
-        fa.of.dst[0] = fs.dst[0] = fa.of.o.dst;
-        fa.of.dst_stride[0] = fs.dst_stride[0] = dst_stride;
-        fa.of.bytes = P->bytes;
-        fa.of.px = fft3d::overlap_add_pixels(fa.of.o, fs, P->bytes);
-        fa.of.o.dst = nullptr;
-        ola_done = true;
-      }
+      ola_done = small && !planes_meet(P, dst, dst_stride, new_src, new_stride) && ola_fuse_setup(P, &of);
+      fa.of = ola_done ? of : fft3d::OlaFuse{};
       {
         const double pix = (double)P->g.W * P->g.H * P->bytes;
         TimeScope ts(P, K_FUSED, pix + (to - from) * S + S + state + (ola_done ? pix : T), st);
@@ -1000,9 +1013,7 @@ int run_filter(fft3d_plane* P, int n, const void* const src[5], const int stride
     news->stamp = ++P->clock;
   }
   if (!g_defer) g_launches++;
-  const bool ints = P->bytes != 4;
-  return output_frame(P, tdom, P->tab, (ints && P->d.is_chroma) ? (float)(1 << (P->d.bits - 1)) : 0.f, dst,
-                      dst_stride, cur, stride ? stride[2] : 0, host, learned, st, ola_done);
+  return output_frame(P, tdom, P->tab, base, dst, dst_stride, cur, stride ? stride[2] : 0, host, learned, st, ola_done);
 }
 
 // A stage for one host-path call, exclusive until the call returns (the
